@@ -4,15 +4,15 @@
 
 namespace dgpu {
 
-// Tiles of 19 x 22 cells, 512 threads, one CTA per SM (126 registers): each
-// phase's items (half states 504, predictor faces 963, corrections 918, final
-// faces 877, updates 418) fill their last round of threads nearly full, where
-// 8 x 32 tiles on 256 threads left rounds of 40 to 124 items in four phases,
-// and the two-cell halo is recomputed on fewer cells per output cell.
-// Measured on the 1024^2 shear layer: 0.486 ms per step against 0.534 ms for
-// 8 x 32 (23 x 18: 0.488, 16 x 26: 0.509, 16 x 32 on 512 threads: 0.549);
-// results bit-identical.
-constexpr int k2dTI = 19, k2dTJ = 22, k2dNT = 512;
+// Tiles of 14 x 26 cells, 256 threads, two CTAs per SM (128 registers, 106 KB
+// each): bound by FP64 issue, so one CTA's barriers, tile load and last rounds
+// of a phase fall under the other's arithmetic. Step time on the 1024^2 shear
+// layer, results bit-identical: 0.288 ms against 0.333 ms for one CTA of 19 x
+// 22 cells on 512 threads (the better shape while the divisions branched:
+// 0.471 against 0.51), 0.312 for 8 x 32, 0.296 for 12 x 30, 0.30 for 16 x 24
+// and 0.33 for three CTAs of 10 x 24 cells on 160 threads; x and y items in
+// one instruction sequence with a runtime direction 0.294.
+constexpr int k2dTI = 14, k2dTJ = 26, k2dNT = 256;
 
 template <int S>
 static int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, const CUtensorMap* map,

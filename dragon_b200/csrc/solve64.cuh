@@ -1,0 +1,561 @@
+// FP64 reconstruction and Riemann solvers of the step kernels on the
+// branch-free divisions of fast64.cuh: the same results as muscl() and
+// face_flux() bit for bit. Each first computes without a branch per division
+// and raises a flag on anything out of the ordinary (an operand out of range,
+// an unphysical or borderline state, a fallback of the solver); the face or
+// cell is then repeated by the plain routine, out of line.
+#pragma once
+
+#include "fast64.cuh"
+#include "recon.cuh"
+#include "riemann.cuh"
+
+namespace dgpu {
+namespace f64 {
+
+// n / d for slopes of one sign (on), 0 otherwise. With n at least 2^-900 the
+// divisor may be smaller than elsewhere.
+__device__ __forceinline__ double slope_quot(double n, double d, bool on, Chk& ck) {
+    const unsigned un = (unsigned)__double2hiint(n) & 0x7fffffffu, ud = (unsigned)__double2hiint(d) & 0x7fffffffu;
+    ck.raise(on && (un - ((1023u - 900u) << 20) >= (1800u << 20) || ud - ((1023u - 450u) << 20) >= (500u << 20)));
+    const double q = div_of(n, on ? d : 1.0);
+    return on ? q : 0.0;
+}
+__device__ __forceinline__ double limit1(int lim, double a, double b, Chk& ck) {
+    switch (lim) {
+        case LIM_MC: return lim_mc(a, b);
+        // the plain form divides (2 a) b by a + b unless a b <= 0
+        case LIM_VANLEER: return slope_quot((2.0 * a) * b, a + b, !(a * b <= 0.0), ck);
+        case LIM_SUPERBEE: return lim_superbee(a, b);
+        case LIM_VANALBADA: return slope_quot((a * b) * (a + b), a * a + b * b, !(a * b <= 0.0), ck);
+        default: return lim_minmod(a, b);
+    }
+}
+
+// TVD::MUSCL with both predicted states physical (else the flag).
+template <bool MHD>
+__device__ __forceinline__ void muscl_body(int lim, const Prim<double>& wL, Prim<double>& outL, const Prim<double>& wC,
+                                           Prim<double>& outR, const Prim<double>& wR, double dt_dL, double dBx,
+                                           double dBy, double dBz, Chk& ck) {
+    Prim<double> dW, L, Rr;
+    dW.rho = f64::limit1(lim, wC.rho - wL.rho, wR.rho - wC.rho, ck);
+    dW.vx = f64::limit1(lim, wC.vx - wL.vx, wR.vx - wC.vx, ck);
+    dW.vy = f64::limit1(lim, wC.vy - wL.vy, wR.vy - wC.vy, ck);
+    dW.vz = f64::limit1(lim, wC.vz - wL.vz, wR.vz - wC.vz, ck);
+    dW.p = f64::limit1(lim, wC.p - wL.p, wR.p - wC.p, ck);
+    L.rho = wC.rho - 0.5 * dW.rho;
+    Rr.rho = wC.rho + 0.5 * dW.rho;
+    L.vx = wC.vx - dW.vx * 0.5;
+    L.vy = wC.vy - dW.vy * 0.5;
+    L.vz = wC.vz - dW.vz * 0.5;
+    Rr.vx = wC.vx + dW.vx * 0.5;
+    Rr.vy = wC.vy + dW.vy * 0.5;
+    Rr.vz = wC.vz + dW.vz * 0.5;
+    L.p = wC.p - 0.5 * dW.p;
+    Rr.p = wC.p + 0.5 * dW.p;
+    if constexpr (MHD) {
+        dW.Bx = f64::limit1(lim, wC.Bx - wL.Bx, wR.Bx - wC.Bx, ck);
+        dW.By = f64::limit1(lim, wC.By - wL.By, wR.By - wC.By, ck);
+        dW.Bz = f64::limit1(lim, wC.Bz - wL.Bz, wR.Bz - wC.Bz, ck);
+        L.Bx = wC.Bx - dW.Bx * 0.5;
+        L.By = wC.By - dW.By * 0.5;
+        L.Bz = wC.Bz - dW.Bz * 0.5;
+        Rr.Bx = wC.Bx + dW.Bx * 0.5;
+        Rr.By = wC.By + dW.By * 0.5;
+        Rr.Bz = wC.Bz + dW.Bz * 0.5;
+    } else {
+        L.Bx = L.By = L.Bz = Rr.Bx = Rr.By = Rr.Bz = 0.0;
+    }
+    ck.pos(L.p);
+    ck.pos(Rr.p);
+    const Cons<double> UL = f64::to_cons<MHD>(L), UR = f64::to_cons<MHD>(Rr);
+    const double pL = f64::pressure<MHD>(UL, rec(UL.rho, ck), ck), pR = f64::pressure<MHD>(UR, rec(UR.rho, ck), ck);
+    Cons<double> corr = c_mul<MHD>(c_sub<MHD>(flux_of<MHD>(UR, pR, Rr.vx, Rr.vy, Rr.vz),
+                                              flux_of<MHD>(UL, pL, L.vx, L.vy, L.vz)), 0.5 * dt_dL);
+    if constexpr (MHD) {
+        const double a_s = (Rr.Bx - L.Bx) * dt_dL;
+        const double vy = 0.5 * (L.vy + Rr.vy), vz = 0.5 * (L.vz + Rr.vz);
+        const double dBy_ = 0.5 * wC.vy * lim_minmod(dBx, -dBy) - 0.5 * vy * a_s;
+        const double dBz_ = 0.5 * wC.vz * lim_minmod(dBx, -dBz) - 0.5 * vz * a_s;
+        corr.By -= dBy_;
+        corr.Bz -= dBz_;
+        corr.E -= k1_4pi * (wC.By * dBy_ + wC.Bz * dBz_);
+    }
+    const Cons<double> oL = c_sub<MHD>(UL, corr), oR = c_sub<MHD>(UR, corr);
+    outL = f64::to_prim<MHD>(oL, rec(oL.rho, ck), ck);
+    outR = f64::to_prim<MHD>(oR, rec(oR.rho, ck), ck);
+    sound_state<MHD>(outL, ck);
+    sound_state<MHD>(outR, ck);
+}
+
+template <bool MHD>
+__device__ __noinline__ bool muscl_plain(int lim, const Prim<double>* w3, Prim<double>* out2, double dt_dL, double dBx,
+                                         double dBy, double dBz) {
+    return dgpu::muscl<MHD>(lim, w3[0], out2[0], w3[1], out2[1], w3[2], dt_dL, dBx, dBy, dBz);
+}
+
+template <bool MHD>
+__device__ __forceinline__ bool muscl(int lim, const Prim<double>& wL, Prim<double>& outL, const Prim<double>& wC,
+                                      Prim<double>& outR, const Prim<double>& wR, double dt_dL, double dBx, double dBy,
+                                      double dBz) {
+    Chk ck;
+    muscl_body<MHD>(lim, wL, outL, wC, outR, wR, dt_dL, dBx, dBy, dBz, ck);
+    if (!ck.bad) return true;
+    const Prim<double> w3[3] = {wL, wC, wR};
+    Prim<double> out2[2];
+    const bool ok = muscl_plain<MHD>(lim, w3, out2, dt_dL, dBx, dBy, dBz);
+    outL = out2[0];
+    outR = out2[1];
+    return ok;
+}
+
+// ---------------------------------------------------------------------------
+// Hydro solvers
+
+struct FaceSide {
+    Rec r;
+    Cons<double> U;
+    double a, sq, h;  // sound speed, sqrt(rho), enthalpy
+};
+__device__ __forceinline__ void face_side(const Prim<double>& w, FaceSide& s, Chk& ck) {
+    ck.pos(w.p);
+    s.r = rec(w.rho, ck);
+    s.U = f64::to_cons<false>(w);
+    s.a = root(quot(kGamma * w.p, s.r), ck);
+    s.sq = root(w.rho, ck);
+}
+// Roe-averaged normal velocity and sound speed (HLL::roeAvg)
+__device__ __forceinline__ void roe_mean(const Prim<double>& L, const Prim<double>& Rt, const FaceSide& sL,
+                                         const FaceSide& sR, double& vx, double& aM, Chk& ck) {
+    const Rec rs = rec(sL.sq + sR.sq, ck);
+    const double _sql = quot(sL.sq, rs), _sqr = quot(sR.sq, rs);
+    const double rho = sL.sq * sR.sq;
+    vx = L.vx * _sql + Rt.vx * _sqr;
+    const double vy = L.vy * _sql + Rt.vy * _sqr, vz = L.vz * _sql + Rt.vz * _sqr;
+    const double hL = quotn(sL.U.E + L.p, sL.r, ck), hR = quotn(sR.U.E + Rt.p, sR.r, ck);
+    const double H = _sql * hL + _sqr * hR;
+    const double a2 = kGm1 * (H - dot3(vx, vy, vz, vx, vy, vz) * 0.5);
+    const double ar = a2 * rho;
+    ck.pos(ar);
+    aM = root(div(kGamma * by_gamma(ar), rho, ck), ck);
+}
+// x-flux of one side's state
+__device__ __forceinline__ Cons<double> side_flux(const Prim<double>& w, const FaceSide& s, Chk& ck) {
+    return flux_of<false>(s.U, f64::pressure<false>(s.U, s.r, ck), w.vx, w.vy, w.vz);
+}
+
+// Riemann::HLLC: one path for the supersonic and the star cases, the flux of
+// the upwind side plus the star part.
+__device__ __forceinline__ Cons<double> hllc(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
+                                             Chk& ck) {
+    face_side(L, sL, ck);
+    face_side(Rt, sR, ck);
+    double vM, aM;
+    roe_mean(L, Rt, sL, sR, vM, aM, ck);
+    const double sl = smin(L.vx - sL.a, vM - aM), sr = smax(Rt.vx + sR.a, vM + aM);
+    const bool out_l = sl >= 0.0, out_r = !out_l && sr <= 0.0;
+    const double mr = Rt.rho * (Rt.vx - sr), ml = L.rho * (L.vx - sl);
+    const double _pr = Rt.p + Rt.rho * Rt.vx * (Rt.vx - sr), _pl = L.p + L.rho * L.vx * (L.vx - sl);
+    double sc = 0.0;
+    const bool star = !(out_l || out_r);
+    if (star) sc = div(_pr - _pl, mr - ml, ck);
+    const bool left = star ? sc > 0.0 : out_l;
+    const Prim<double> X = left ? L : Rt;
+    const FaceSide S = left ? sL : sR;
+    Cons<double> F = side_flux(X, S, ck);
+    if (star) {
+        const double sx = left ? sl : sr;
+        const double w = sx - X.vx;
+        const Rec rd = rec(sx - sc, ck);
+        Cons<double> U;
+        const double rw = S.U.rho * w;
+        U.rho = quotn(rw, rd, ck);
+        U.E = quotn(S.U.E * w, rd, ck);
+        U.my = S.U.my * w;
+        U.mz = S.U.mz * w;
+        quots(rd, ck, U.my, U.mz);
+        U.Bx = U.By = U.Bz = 0;
+        U.mx = U.rho * sc;
+        U.E += U.rho * (sc - X.vx) * (sc + div(X.p, rw, ck));
+        F = c_add<false>(F, c_mul<false>(c_sub<false>(U, S.U), sx));
+    }
+    return F;
+}
+
+// Riemann::HLL(SL, SR)
+__device__ __forceinline__ Cons<double> hll_speeds(const Prim<double>& L, const Prim<double>& Rt, const FaceSide& sL,
+                                                   const FaceSide& sR, double sl, double sr, Chk& ck) {
+    const Cons<double> FL = side_flux(L, sL, ck), FR = side_flux(Rt, sR, ck);
+    if (sl >= 0.0) return FL;
+    if (sr <= 0.0) return FR;
+    const Cons<double> n = c_add<false>(c_sub<false>(c_mul<false>(FL, sr), c_mul<false>(FR, sl)),
+                                        c_mul<false>(c_sub<false>(sR.U, sL.U), sl * sr));
+    Cons<double> F = n;
+    quots(rec(sr - sl, ck), ck, F.rho, F.E, F.mx, F.my, F.mz);
+    return F;
+}
+__device__ __forceinline__ Cons<double> hll(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
+                                            Chk& ck) {
+    face_side(L, sL, ck);
+    face_side(Rt, sR, ck);
+    double vM, aM;
+    roe_mean(L, Rt, sL, sR, vM, aM, ck);
+    return hll_speeds(L, Rt, sL, sR, smin(L.vx - sL.a, vM - aM), smax(Rt.vx + sR.a, vM + aM), ck);
+}
+__device__ __forceinline__ Cons<double> hlle(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
+                                             Chk& ck) {
+    face_side(L, sL, ck);
+    face_side(Rt, sR, ck);
+    const double sql = sL.sq, sqr = sR.sq, aL = sL.a, aR = sR.a;
+    const Rec rs = rec(sql + sqr, ck);
+    const double _sql = quot(sql, rs), _sqr = quot(sqr, rs);
+    const double _v = quotn(Rt.vx - L.vx, rs, ck);
+    double d = (_sql * aL * aL + _sqr * aR * aR) + 0.5 * (sql * sqr) * _v * _v;
+    d = root(d, ck);
+    const double u = _sql * L.vx + _sqr * Rt.vx;
+    return hll_speeds(L, Rt, sL, sR, smin(L.vx - aL, u - d), smax(Rt.vx + aR, u + d), ck);
+}
+
+// Riemann::Roe with the Harten-Hyman fix; the two entropy-fix returns raise
+// the flag (transonic rarefactions are few).
+__device__ __forceinline__ Cons<double> roe(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
+                                            Chk& ck) {
+    face_side(L, sL, ck);
+    face_side(Rt, sR, ck);
+    const Rec rs = rec(sL.sq + sR.sq, ck);
+    const double _sql = quot(sL.sq, rs), _sqr = quot(sR.sq, rs);
+    const double _rho = sL.sq * sR.sq;
+    const double vx = L.vx * _sql + Rt.vx * _sqr, vy = L.vy * _sql + Rt.vy * _sqr, vz = L.vz * _sql + Rt.vz * _sqr;
+    const double _H = _sql * quotn(sL.U.E + L.p, sL.r, ck) + _sqr * quotn(sR.U.E + Rt.p, sR.r, ck);
+    const double V2 = dot3(vx, vy, vz, vx, vy, vz);
+    const double _a = root(kGm1 * (_H - V2 * 0.5), ck);
+    const double dp = Rt.p - L.p, ra = _rho * _a, du = Rt.vx - L.vx;
+    // (2 a) a is exactly twice a a, so all three quotients share 1 / (a a)
+    const Rec r2 = rec(_a * _a, ck);
+    double q0 = dp - ra * du, q1 = dp, q4 = dp + ra * du;
+    quots(r2, ck, q0, q1, q4);
+    const double al0 = 0.5 * q0, al1 = (Rt.rho - L.rho) - q1, al2 = _rho * (Rt.vy - L.vy), al3 = _rho * (Rt.vz - L.vz),
+                 al4 = 0.5 * q4;
+    const Cons<double> K0{1.0, _H - vx * _a, vx - _a, vy - 0.0, vz - 0.0, 0, 0, 0};
+    const Cons<double> K4{1.0, _H + vx * _a, vx + _a, vy + 0.0, vz + 0.0, 0, 0, 0};
+    {
+        const Cons<double> SL = c_add<false>(sL.U, c_mul<false>(K0, al0));
+        const Rec r = rec(SL.rho, ck);
+        const double aSL = root(quotn(kGamma * f64::pressure<false>(SL, r, ck), r, ck), ck);
+        ck.raise(L.vx - sL.a < 0.0 && quotn(SL.mx, r, ck) - aSL > 0.0);
+        const Cons<double> SR = c_sub<false>(sR.U, c_mul<false>(K4, al4));
+        const Rec q = rec(SR.rho, ck);
+        const double aSR = root(quotn(kGamma * f64::pressure<false>(SR, q, ck), q, ck), ck);
+        ck.raise(Rt.vx + sR.a > 0.0 && quotn(SR.mx, q, ck) + aSR < 0.0);
+    }
+    Cons<double> F = c_add<false>(side_flux(L, sL, ck), side_flux(Rt, sR, ck));
+    const Cons<double> K1{1.0, V2 * 0.5, vx, vy, vz, 0, 0, 0}, K2{0.0, vy, 0.0, 1.0, 0.0, 0, 0, 0},
+        K3{0.0, vz, 0.0, 0.0, 1.0, 0, 0, 0};
+    F = c_sub<false>(F, c_mul<false>(K0, al0 * fabs(vx - _a)));
+    F = c_sub<false>(F, c_mul<false>(K1, al1 * fabs(vx)));
+    F = c_sub<false>(F, c_mul<false>(K2, al2 * fabs(vx)));
+    F = c_sub<false>(F, c_mul<false>(K3, al3 * fabs(vx)));
+    F = c_sub<false>(F, c_mul<false>(K4, al4 * fabs(vx + _a)));
+    return c_mul<false>(F, 0.5);
+}
+
+// ---------------------------------------------------------------------------
+// MHD solvers. The normal field is averaged into both sides first, as the
+// plain routines do.
+
+struct MhdSide {
+    Rec r;        // of the density
+    double E, c;  // energy, fast speed along x
+};
+__device__ __forceinline__ void mhd_side(const Prim<double>& w, MhdSide& s, Chk& ck) {
+    s.r = rec(w.rho, ck);
+    s.c = f64::fast_speed(w, w.Bx, s.r, ck);
+    s.E = f64::energy<true>(w);
+}
+__device__ __forceinline__ Cons<double> mhd_cons(const Prim<double>& w, const MhdSide& s) {
+    return Cons<double>{w.rho, s.E, w.vx * w.rho, w.vy * w.rho, w.vz * w.rho, w.Bx, w.By, w.Bz};
+}
+__device__ __forceinline__ Cons<double> mhd_flux(const Prim<double>& w, const MhdSide& s, Chk& ck) {
+    const Cons<double> U = mhd_cons(w, s);
+    return flux_of<true>(U, f64::pressure<true>(U, s.r, ck), w.vx, w.vy, w.vz);
+}
+__device__ __forceinline__ double b2_of(const Prim<double>& w) { return dot3(w.Bx, w.By, w.Bz, w.Bx, w.By, w.Bz); }
+
+// The state behind one outer wave: its velocity and field, and with FLUX its
+// conservative state and flux. d: SK - SM and its reciprocal; ZERO: the branch
+// without a normal field.
+struct MhdStar {
+    Cons<double> u, F;
+    Prim<double> w;
+};
+template <bool ZERO, bool FLUX>
+__device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s, double x, double SK, double SM,
+                                         const Rec& d, double rho, double pT, double Bx, MhdStar& o, Chk& ck) {
+    Cons<double> u;
+    u.rho = rho;
+    double vy, vz;
+    if constexpr (ZERO) {
+        ck.raise(!(fabs(d.b) >= 1e-12));
+        const double num = SK - K.vx;
+        u.Bx = 0;
+        u.By = K.By * num;
+        u.Bz = K.Bz * num;
+        quots(d, ck, u.By, u.Bz);
+        vy = K.vy;
+        vz = K.vz;
+    } else {
+        const double bb = (Bx * Bx) * k1_4pi;
+        const double den = x * d.b - bb, num = x * (SK - K.vx) - bb, dv = SM - K.vx;
+        ck.raise(!(fabs(den) >= 1e-12));
+        const Rec q = rec(den, ck);
+        u.Bx = Bx;
+        u.By = K.By * num;
+        u.Bz = K.Bz * num;
+        double ty = (K.By * Bx) * dv, tz = (K.Bz * Bx) * dv;
+        quots(q, ck, u.By, u.Bz, ty, tz);
+        vy = K.vy - ty * k1_4pi;
+        vz = K.vz - tz * k1_4pi;
+    }
+    u.mx = SM * u.rho;
+    u.my = vy * u.rho;
+    u.mz = vz * u.rho;
+    double E = s.E * (SK - K.vx);
+    E += pT * SM - (K.p + b2_of(K) * k1_8pi) * K.vx;
+    if constexpr (!ZERO)
+        E += Bx * (dot3(K.vx, K.vy, K.vz, K.Bx, K.By, K.Bz) - dot3(SM, vy, vz, u.Bx, u.By, u.Bz)) * k1_4pi;
+    u.E = quotn(E, d, ck);
+    ck.pos(u.E);
+    const Rec q = rec(u.rho, ck);
+    Prim<double> w;
+    w.rho = u.rho;
+    w.vx = u.mx;
+    w.vy = u.my;
+    w.vz = u.mz;
+    quots(q, ck, w.vx, w.vy, w.vz);
+    w.Bx = u.Bx;
+    w.By = u.By;
+    w.Bz = u.Bz;
+    w.p = pT - b2_of(w) * k1_8pi;
+    sound_state<true>(w, ck);
+    if constexpr (!ZERO) surely_physical<true>(u, ck);
+    o.w = w;
+    o.u = u;
+    if constexpr (FLUX) {
+        o.F = c_add<true>(mhd_flux(K, s, ck), c_mul<true>(c_sub<true>(u, mhd_cons(K, s)), SK));
+        o.F.Bx = 0;
+    }
+}
+
+// Riemann::HLLD and HLLD_zero_B; an unphysical star state (their way to HLLE)
+// raises the flag. Only the side the contact leaves behind needs its star flux
+// and energy (SsL >= 0 implies SM >= 0, SsR <= 0 implies SM <= 0), so the
+// other side's star state comes first and leaves its velocity and field:
+// fewer values alive at a time (both sides whole spilled 700 bytes).
+__device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, Chk& ck) {
+    const double Bx = (L.Bx + Rt.Bx) * 0.5;
+    L.Bx = Bx;
+    Rt.Bx = Bx;
+    MhdSide sL, sR;
+    mhd_side(L, sL, ck);
+    mhd_side(Rt, sR, ck);
+    const double SL = smin(L.vx - sL.c, Rt.vx - sR.c);
+    const double SR = smax(L.vx + sL.c, Rt.vx + sR.c);
+    const bool outer = SL >= 0.0 || SR <= 0.0;
+    double SM = SL >= 0.0 ? 1.0 : -1.0, pT = 0.0, xL = 0.0, xR = 0.0;
+    if (!outer) {
+        const double pTL = L.p + b2_of(L) * k1_8pi, pTR = Rt.p + b2_of(Rt) * k1_8pi;
+        xL = L.rho * (SL - L.vx);
+        xR = Rt.rho * (SR - Rt.vx);
+        const Rec rx = rec(xR - xL, ck);
+        SM = (xR * Rt.vx - xL * L.vx) - (pTR - pTL);
+        quots(rx, ck, SM);
+        pT = quotn(xR * pTL - xL * pTR + xL * xR * (Rt.vx - L.vx), rx, ck);
+    }
+    const bool left = SM >= 0.0;
+    const Prim<double> K = left ? L : Rt;
+    const MhdSide sK = left ? sL : sR;
+    if (outer) return mhd_flux(K, sK, ck);
+    const double cutoff = smax(b2_of(L) + b2_of(Rt), 1e-100);
+    const bool zero = Bx * Bx < 1e-12 * cutoff || Bx == 0.0;
+    const Prim<double> O = left ? Rt : L;
+    const MhdSide sO = left ? sR : sL;
+    const double SK = left ? SL : SR, SO = left ? SR : SL, xK = left ? xL : xR, xO = left ? xR : xL;
+    const Rec dK = rec(SK - SM, ck), dO = rec(SO - SM, ck);
+    const double rhoK = quotn(xK, dK, ck), rhoO = quotn(xO, dO, ck);
+    MhdStar k, o;
+    if (zero) {
+        mhd_star<true, true>(K, sK, xK, SK, SM, dK, rhoK, pT, Bx, k, ck);
+        if (SM != 0.0) return k.F;
+        mhd_star<true, true>(O, sO, xO, SO, SM, dO, rhoO, pT, Bx, o, ck);
+        const double sql = root(rhoK, ck), sqr = root(rhoO, ck);
+        const Rec q = rec(sql + sqr, ck);
+        return c_add<true>(c_mul<true>(k.F, quot(sql, q)), c_mul<true>(o.F, quot(sqr, q)));
+    }
+    const double sqK = root(rhoK, ck), sqO = root(rhoO, ck);
+    const double ab = fabs(Bx), s4 = sq4pi();
+    const double aK = div(ab, s4 * sqK, ck), aO = div(ab, s4 * sqO, ck);
+    const double SsL = SM - (left ? aK : aO), SsR = SM + (left ? aO : aK);
+    const bool inner = !(SsL >= 0.0) && !(SsR <= 0.0);
+    if (inner) mhd_star<false, false>(O, sO, xO, SO, SM, dO, rhoO, pT, Bx, o, ck);
+    mhd_star<false, true>(K, sK, xK, SK, SM, dK, rhoK, pT, Bx, k, ck);
+    ck.raise(SsL >= 0.0 ? !left : SsR <= 0.0 && left);
+    if (!inner) return k.F;
+    const double lvy = left ? k.w.vy : o.w.vy, lvz = left ? k.w.vz : o.w.vz, rvy = left ? o.w.vy : k.w.vy,
+                 rvz = left ? o.w.vz : k.w.vz, lBy = left ? k.w.By : o.w.By, lBz = left ? k.w.Bz : o.w.Bz,
+                 rBy = left ? o.w.By : k.w.By, rBz = left ? o.w.Bz : k.w.Bz, sqL = left ? sqK : sqO,
+                 sqR = left ? sqO : sqK;
+    const Rec q = rec(sqL + sqR, ck);
+    const double _sqL = quot(sqL, q), _sqR = quot(sqR, q);
+    const double sbx = Bx > 0.0 ? s4 : -s4;
+    Prim<double> w;
+    w.rho = rhoK;
+    w.vx = SM;
+    double tvy = (rBy - lBy) * sbx * k1_4pi, tvz = (rBz - lBz) * sbx * k1_4pi, tBy = (rvy - lvy) * sbx * sqL * sqR,
+           tBz = (rvz - lvz) * sbx * sqL * sqR;
+    quots(q, ck, tvy, tvz, tBy, tBz);
+    w.vy = (lvy * _sqL + rvy * _sqR) + tvy;
+    w.vz = (lvz * _sqL + rvz * _sqR) + tvz;
+    w.Bx = Bx;
+    w.By = (rBy * _sqL + lBy * _sqR) + tBy;
+    w.Bz = (rBz * _sqL + lBz * _sqR) + tBz;
+    const double dE = sbx * (dot3(k.w.vx, k.w.vy, k.w.vz, k.w.Bx, k.w.By, k.w.Bz) -
+                             dot3(w.vx, w.vy, w.vz, w.Bx, w.By, w.Bz)) * k1_4pi * sqK;
+    const Cons<double> u{rhoK, left ? k.u.E - dE : k.u.E + dE, w.vx * rhoK, w.vy * rhoK, w.vz * rhoK, w.Bx, w.By, w.Bz};
+    w.p = pT - b2_of(w) * k1_8pi;
+    sound_state<true>(w, ck);
+    ck.fin(u.E);
+    ck.fin(u.mx);
+    ck.fin(u.my);
+    ck.fin(u.mz);
+    return c_add<true>(k.F, c_mul<true>(c_sub<true>(u, k.u), left ? SsL : SsR));
+}
+
+// Riemann::HLLE for MHD states
+__device__ __forceinline__ Cons<double> hlle_mhd(Prim<double> L, Prim<double> Rt, Chk& ck) {
+    const double Bx = (L.Bx + Rt.Bx) * 0.5;
+    L.Bx = Bx;
+    Rt.Bx = Bx;
+    MhdSide sL, sR;
+    mhd_side(L, sL, ck);
+    mhd_side(Rt, sR, ck);
+    const double sql = root(L.rho, ck), sqr = root(Rt.rho, ck), aL = sL.c, aR = sR.c;
+    const Rec rs = rec(sql + sqr, ck);
+    const double _sql = quot(sql, rs), _sqr = quot(sqr, rs);
+    const double _v = quotn(Rt.vx - L.vx, rs, ck);
+    const double d = root((_sql * aL * aL + _sqr * aR * aR) + 0.5 * (sql * sqr) * _v * _v, ck);
+    const double u = _sql * L.vx + _sqr * Rt.vx;
+    const double sl = smin(L.vx - aL, u - d), sr = smax(Rt.vx + aR, u + d);
+    const Cons<double> FL = mhd_flux(L, sL, ck), FR = mhd_flux(Rt, sR, ck);
+    if (sl >= 0.0) return FL;
+    if (sr <= 0.0) return FR;
+    const Cons<double> n = c_add<true>(c_sub<true>(c_mul<true>(FL, sr), c_mul<true>(FR, sl)),
+                                       c_mul<true>(c_sub<true>(mhd_cons(Rt, sR), mhd_cons(L, sL)), sl * sr));
+    Cons<double> F = n;
+    quots(rec(sr - sl, ck), ck, F.rho, F.E, F.mx, F.my, F.mz, F.Bx, F.By, F.Bz);
+    return F;
+}
+
+template <bool MHD, int SOLVER>
+__device__ __noinline__ bool face_plain(const Prim<double>* LR, double dt_dx, const ExactOpts* eo, Cons<double>* F,
+                                        FaceStats* st) {
+    return face_flux_x<MHD, SOLVER, double>(LR[0], LR[1], dt_dx, *eo, *F, st);
+}
+
+// The flux along x of the states on both sides of a face, as face_flux_x. The
+// exact solver is pow and MHD HLL is rare: they take the plain routine.
+template <bool MHD, int SOLVER>
+__device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
+                                            const ExactOpts& eo, Cons<double>& F, FaceStats* st) {
+    if constexpr (MHD ? SOLVER == RS_HLL : SOLVER == RS_EXACT) {
+        return dgpu::face_flux_x<MHD, SOLVER>(L, Rt, dt_dL, eo, F, st);
+    } else {
+        Chk ck;
+        if constexpr (MHD) {
+            if constexpr (SOLVER == RS_HLLE) F = hlle_mhd(L, Rt, ck);
+            else F = hlld(L, Rt, ck);
+        } else {
+            FaceSide sL, sR;
+            if constexpr (SOLVER == RS_HLL) F = hll(L, Rt, sL, sR, ck);
+            else if constexpr (SOLVER == RS_HLLE) F = hlle(L, Rt, sL, sR, ck);
+            else if constexpr (SOLVER == RS_ROE) F = roe(L, Rt, sL, sR, ck);
+            else F = hllc(L, Rt, sL, sR, ck);
+            // verify_and_fallback (Flux.cpp:77-97)
+            if (dt_dL > 0.0) {
+                surely_physical<false>(c_sub<false>(sL.U, c_mul<false>(F, dt_dL)), ck);
+                surely_physical<false>(c_add<false>(sR.U, c_mul<false>(F, dt_dL)), ck);
+            }
+        }
+        if (!ck.bad) return true;
+        const Prim<double> LR[2] = {L, Rt};
+        Cons<double> G;
+        const ExactOpts e = eo;
+        FaceStats s = *st;
+        const bool ok = face_plain<MHD, SOLVER>(LR, dt_dL, &e, &G, &s);
+        *st = s;
+        F = G;
+        return ok;
+    }
+}
+template <bool MHD, int SOLVER, int AX>
+__device__ __forceinline__ bool face_flux(Prim<double> L, Prim<double> Rt, double dt_dL, const ExactOpts& eo,
+                                          Cons<double>& F, FaceStats* st) {
+    swap_axis<AX>(L);
+    swap_axis<AX>(Rt);
+    const bool ok = f64::face_flux_x<MHD, SOLVER>(L, Rt, dt_dL, eo, F, st);
+    swap_axis<AX>(F);
+    return ok;
+}
+
+// ---------------------------------------------------------------------------
+// The conservative update of a cell
+
+// protect_thermal's gate 8 pi p / B^2 <= 0.1 without the division, the flag
+// where the rounded quotient could fall on either side.
+__device__ __forceinline__ bool keeps_thermal(const Prim<double>& w, int mode, Chk& ck) {
+    if (mode == 0) return false;
+    if (mode == 1) return true;
+    const double B2 = b2_of(w);
+    const double n = k8pi * w.p, t = 0.1 * B2;
+    ck.fin(B2);
+    const bool under = n < t * (1.0 - 0x1p-48);
+    ck.raise(!under && !(n > t * (1.0 + 0x1p-48)));
+    return under && B2 != 0.0;
+}
+// computeBodyField (B_fields.cpp:70-79): the cell with its field replaced, r
+// the reciprocal of its density.
+__device__ __forceinline__ Prim<double> body_field(Prim<double> w, double bx, double by, double bz, int mode,
+                                                   const Rec& r, Chk& ck) {
+    const bool keep = keeps_thermal(w, mode, ck);
+    ck.pos(w.p);
+    Cons<double> U = f64::to_cons<true>(w);
+    U.Bx = bx; U.By = by; U.Bz = bz;
+    const Prim<double> n = f64::to_prim<true>(U, r, ck);
+    w.Bx = bx; w.By = by; w.Bz = bz;
+    return keep ? w : n;
+}
+
+// A half state w plus its transverse correction d, with the normal field
+// (component ax) replaced by b.
+static __device__ __noinline__ void corrected_mhd_plain(Prim<double>* w, const Cons<double>* d, int ax, double b) {
+    Cons<double> u = dgpu::c_add<true>(dgpu::to_cons<true>(*w), *d);
+    (ax == 0 ? u.Bx : ax == 1 ? u.By : u.Bz) = b;
+    *w = dgpu::to_prim<true>(u);
+}
+template <int AX>
+__device__ __forceinline__ Prim<double> corrected_mhd(const Prim<double>& w, const Cons<double>& d, double b) {
+    Chk ck;
+    ck.pos(w.p);
+    Cons<double> u = c_add<true>(f64::to_cons<true>(w), d);
+    (AX == 0 ? u.Bx : AX == 1 ? u.By : u.Bz) = b;
+    Prim<double> r = f64::to_prim<true>(u, rec(u.rho, ck), ck);
+    if (ck.bad) {
+        Prim<double> t = w;
+        const Cons<double> e = d;
+        corrected_mhd_plain(&t, &e, AX, b);
+        r = t;
+    }
+    return r;
+}
+
+}  // namespace f64
+}  // namespace dgpu

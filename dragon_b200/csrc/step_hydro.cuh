@@ -12,6 +12,7 @@
 #include "grid.cuh"
 #include "recon.cuh"
 #include "riemann.cuh"
+#include "update64.cuh"
 #include "tma.cuh"
 
 namespace dgpu {
@@ -139,12 +140,12 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
         };
         const Prim<double> wc = W(a + 1, b + 1);
         Prim<double> oL, oR;
-        first_order += !muscl<false>(sa.limiter, W(a, b + 1), oL, wc, oR, W(a + 2, b + 1), dt_dx, 0.0, 0.0, 0.0);
+        first_order += !f64::muscl<false>(sa.limiter, W(a, b + 1), oL, wc, oR, W(a + 2, b + 1), dt_dx, 0.0, 0.0, 0.0);
         hs_put(S, HS_XL, a, b, oL);
         hs_put(S, HS_XR, a, b, oR);
         Prim<double> yl = W(a + 1, b), yc = wc, yr = W(a + 1, b + 2);
         swap_xy(yl); swap_xy(yc); swap_xy(yr);
-        first_order += !muscl<false>(sa.limiter, yl, oL, yc, oR, yr, dt_dy, 0.0, 0.0, 0.0);
+        first_order += !f64::muscl<false>(sa.limiter, yl, oL, yc, oR, yr, dt_dy, 0.0, 0.0, 0.0);
         swap_xy(oL); swap_xy(oR);
         hs_put(S, HS_YL, a, b, oL);
         hs_put(S, HS_YR, a, b, oR);
@@ -160,7 +161,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             const int a = t / (TJ + 2), b = t % (TJ + 2);
             const int i = i0 + a, j = j0 - 1 + b;
             if (!(i <= nx && j >= -1 && j <= ny)) continue;
-            bool ok = face_flux<false, SOLVER, 0>(hs_get(S, HS_XR, a, b), hs_get(S, HS_XL, a + 1, b), dt_dx, eo, F, &st);
+            bool ok = f64::face_flux<false, SOLVER, 0>(hs_get(S, HS_XR, a, b), hs_get(S, HS_XL, a + 1, b), dt_dx, eo, F, &st);
             if (!ok) record_error(ctl, ST_PRELIM_FLUX, (long long)(i + g) * (ny + 2 * g) + (j + g));
             S.u.f.fx[0][a][b] = F.rho; S.u.f.fx[1][a][b] = F.E; S.u.f.fx[2][a][b] = F.mx;
             S.u.f.fx[3][a][b] = F.my; S.u.f.fx[4][a][b] = F.mz;
@@ -169,7 +170,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             const int a = q / (TJ + 1), b = q % (TJ + 1);
             const int i = i0 - 1 + a, j = j0 + b;
             if (!(i >= -1 && i <= nx && j <= ny)) continue;
-            bool ok = face_flux<false, SOLVER, 1>(hs_get(S, HS_YR, a, b), hs_get(S, HS_YL, a, b + 1), dt_dy, eo, F, &st);
+            bool ok = f64::face_flux<false, SOLVER, 1>(hs_get(S, HS_YR, a, b), hs_get(S, HS_YL, a, b + 1), dt_dy, eo, F, &st);
             if (!ok) record_error(ctl, ST_PRELIM_FLUX, (long long)(i + g) * (ny + 2 * g) + (j + g));
             S.u.f.fy[0][a][b] = F.rho; S.u.f.fy[1][a][b] = F.E; S.u.f.fy[2][a][b] = F.mx;
             S.u.f.fy[3][a][b] = F.my; S.u.f.fy[4][a][b] = F.mz;
@@ -190,8 +191,8 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             tr.mx = (S.u.f.fy[2][a][b] - S.u.f.fy[2][a][b - 1]) * hdy;
             tr.my = (S.u.f.fy[3][a][b] - S.u.f.fy[3][a][b - 1]) * hdy;
             tr.mz = (S.u.f.fy[4][a][b] - S.u.f.fy[4][a][b - 1]) * hdy;
-            hs_put(S, HS_XL, a, b, to_prim<false>(c_sub<false>(to_cons<false>(hs_get(S, HS_XL, a, b)), tr)));
-            hs_put(S, HS_XR, a, b, to_prim<false>(c_sub<false>(to_cons<false>(hs_get(S, HS_XR, a, b)), tr)));
+            hs_put(S, HS_XL, a, b, f64::corrected<false>(hs_get(S, HS_XL, a, b), tr));
+            hs_put(S, HS_XR, a, b, f64::corrected<false>(hs_get(S, HS_XR, a, b), tr));
         } else {
             const int q = t - NCX;
             const int a = q / HJ + 1, b = q % HJ;
@@ -203,8 +204,8 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             tr.mx = (S.u.f.fx[2][a][b] - S.u.f.fx[2][a - 1][b]) * hdx;
             tr.my = (S.u.f.fx[3][a][b] - S.u.f.fx[3][a - 1][b]) * hdx;
             tr.mz = (S.u.f.fx[4][a][b] - S.u.f.fx[4][a - 1][b]) * hdx;
-            hs_put(S, HS_YL, a, b, to_prim<false>(c_sub<false>(to_cons<false>(hs_get(S, HS_YL, a, b)), tr)));
-            hs_put(S, HS_YR, a, b, to_prim<false>(c_sub<false>(to_cons<false>(hs_get(S, HS_YR, a, b)), tr)));
+            hs_put(S, HS_YL, a, b, f64::corrected<false>(hs_get(S, HS_YL, a, b), tr));
+            hs_put(S, HS_YR, a, b, f64::corrected<false>(hs_get(S, HS_YR, a, b), tr));
         }
     }
     __syncthreads();
@@ -217,7 +218,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             const int a = t / TJ, b = t % TJ;
             const int i = i0 + a, j = j0 + b;
             if (!(i <= nx && j < ny)) continue;
-            bool ok = face_flux<false, SOLVER, 0>(hs_get(S, HS_XR, a, b + 1), hs_get(S, HS_XL, a + 1, b + 1), dt_dx, eo, F, &st);
+            bool ok = f64::face_flux<false, SOLVER, 0>(hs_get(S, HS_XR, a, b + 1), hs_get(S, HS_XL, a + 1, b + 1), dt_dx, eo, F, &st);
             if (!ok) record_error(ctl, ST_FINAL_FLUX, (long long)(i + g) * (ny + 2 * g) + (j + g));
             S.u.f.fx[0][a][b + 1] = F.rho; S.u.f.fx[1][a][b + 1] = F.E; S.u.f.fx[2][a][b + 1] = F.mx;
             S.u.f.fx[3][a][b + 1] = F.my; S.u.f.fx[4][a][b + 1] = F.mz;
@@ -226,7 +227,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
             const int a = q / (TJ + 1), b = q % (TJ + 1);
             const int i = i0 + a, j = j0 + b;
             if (!(i < nx && j <= ny)) continue;
-            bool ok = face_flux<false, SOLVER, 1>(hs_get(S, HS_YR, a + 1, b), hs_get(S, HS_YL, a + 1, b + 1), dt_dy, eo, F, &st);
+            bool ok = f64::face_flux<false, SOLVER, 1>(hs_get(S, HS_YR, a + 1, b), hs_get(S, HS_YL, a + 1, b + 1), dt_dy, eo, F, &st);
             if (!ok) record_error(ctl, ST_FINAL_FLUX, (long long)(i + g) * (ny + 2 * g) + (j + g));
             S.u.f.fy[0][a + 1][b] = F.rho; S.u.f.fy[1][a + 1][b] = F.E; S.u.f.fy[2][a + 1][b] = F.mx;
             S.u.f.fy[3][a + 1][b] = F.my; S.u.f.fy[4][a + 1][b] = F.mz;
@@ -237,31 +238,28 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
     // P5: conservative update, finiteness / physicality, CFL speed of the new state
     // (applyFluxes, Unsplit.cpp:256-270, and the check at Unsplit.cpp:95-99)
     double vmax = 0.0;
+    const f64::Widths wd = f64::widths(2, sa.dx, sa.dy, 0.0);
     for (int t = threadIdx.x; t < TI * TJ; t += NT) {
         const int a = t / TJ, b = t % TJ;
         const int i = i0 + a, j = j0 + b;
         if (!(i < nx && j < ny)) continue;
         const long long m = gidx2(G, i, j);
-        Prim<double> w0 = load_prim<false>(win, PL, m);
-        Cons<double> U = to_cons<false>(w0);
-        Cons<double> d;
-        d.rho = (S.u.f.fx[0][a][b + 1] - S.u.f.fx[0][a + 1][b + 1]) * dt_dx;
-        d.E = (S.u.f.fx[1][a][b + 1] - S.u.f.fx[1][a + 1][b + 1]) * dt_dx;
-        d.mx = (S.u.f.fx[2][a][b + 1] - S.u.f.fx[2][a + 1][b + 1]) * dt_dx;
-        d.my = (S.u.f.fx[3][a][b + 1] - S.u.f.fx[3][a + 1][b + 1]) * dt_dx;
-        d.mz = (S.u.f.fx[4][a][b + 1] - S.u.f.fx[4][a + 1][b + 1]) * dt_dx;
-        U = c_add<false>(U, d);
-        d.rho = (S.u.f.fy[0][a + 1][b] - S.u.f.fy[0][a + 1][b + 1]) * dt_dy;
-        d.E = (S.u.f.fy[1][a + 1][b] - S.u.f.fy[1][a + 1][b + 1]) * dt_dy;
-        d.mx = (S.u.f.fy[2][a + 1][b] - S.u.f.fy[2][a + 1][b + 1]) * dt_dy;
-        d.my = (S.u.f.fy[3][a + 1][b] - S.u.f.fy[3][a + 1][b + 1]) * dt_dy;
-        d.mz = (S.u.f.fy[4][a + 1][b] - S.u.f.fy[4][a + 1][b + 1]) * dt_dy;
-        U = c_add<false>(U, d);
-        Prim<double> nw = to_prim<false>(U);
-        if (!is_finite<false>(U)) record_error(ctl, ST_NAN, (long long)(i + g) * (ny + 2 * g) + (j + g));
-        else if (!is_physical<false>(nw)) record_error(ctl, ST_UNPHYSICAL, (long long)(i + g) * (ny + 2 * g) + (j + g));
-        store_prim<false>(wout, PL, m, nw);
-        vmax = speed_max(vmax, cfl_speed<false>(nw, sa.cfl, sa.dx, sa.dy, 0.0));
+        const Prim<double> w0 = load_prim<false>(win, PL, m);
+        Cons<double> dX, dY;
+        dX.rho = (S.u.f.fx[0][a][b + 1] - S.u.f.fx[0][a + 1][b + 1]) * dt_dx;
+        dX.E = (S.u.f.fx[1][a][b + 1] - S.u.f.fx[1][a + 1][b + 1]) * dt_dx;
+        dX.mx = (S.u.f.fx[2][a][b + 1] - S.u.f.fx[2][a + 1][b + 1]) * dt_dx;
+        dX.my = (S.u.f.fx[3][a][b + 1] - S.u.f.fx[3][a + 1][b + 1]) * dt_dx;
+        dX.mz = (S.u.f.fx[4][a][b + 1] - S.u.f.fx[4][a + 1][b + 1]) * dt_dx;
+        dY.rho = (S.u.f.fy[0][a + 1][b] - S.u.f.fy[0][a + 1][b + 1]) * dt_dy;
+        dY.E = (S.u.f.fy[1][a + 1][b] - S.u.f.fy[1][a + 1][b + 1]) * dt_dy;
+        dY.mx = (S.u.f.fy[2][a + 1][b] - S.u.f.fy[2][a + 1][b + 1]) * dt_dy;
+        dY.my = (S.u.f.fy[3][a + 1][b] - S.u.f.fy[3][a + 1][b + 1]) * dt_dy;
+        dY.mz = (S.u.f.fy[4][a + 1][b] - S.u.f.fy[4][a + 1][b + 1]) * dt_dy;
+        const f64::Updated r = f64::updated<false>(w0, sa, wd, dX, dY);
+        if (r.stage) record_error(ctl, r.stage, (long long)(i + g) * (ny + 2 * g) + (j + g));
+        store_prim<false>(wout, PL, m, r.w);
+        vmax = speed_max(vmax, r.speed);
     }
     copy_ghosts_2d<5>(G, win, wout, i0, j0, TI, TJ);
 
@@ -344,7 +342,7 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
         const int p = p0 - 1 + q;
         if (p >= 1 && p <= np - 2) {
             Prim<double> oL, oR;
-            first_order += !muscl<MHD>(sa.limiter, getw(q), oL, getw(q + 1), oR, getw(q + 2), dt_dx, 0.0, 0.0, 0.0);
+            first_order += !f64::muscl<MHD>(sa.limiter, getw(q), oL, getw(q + 1), oR, getw(q + 2), dt_dx, 0.0, 0.0, 0.0);
             put(sL, q, oL);
             put(sR, q, oR);
         }
@@ -357,18 +355,21 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
         Prim<double> L = (p == 0) ? getw(q + 1) : get(sR, q);
         Prim<double> Rt = (p + 1 == np - 1) ? getw(q + 2) : get(sL, q + 1);
         Cons<double> F;
-        bool ok = face_flux<MHD, SOLVER, 0>(L, Rt, dt_dx, eo, F, &st);
+        bool ok = f64::face_flux<MHD, SOLVER, 0>(L, Rt, dt_dx, eo, F, &st);
         if (!ok) record_error(ctl, ST_FINAL_FLUX, p);
         sF[0][q] = F.rho; sF[1][q] = F.E; sF[2][q] = F.mx; sF[3][q] = F.my; sF[4][q] = F.mz;
         if constexpr (MHD) { sF[5][q] = F.Bx; sF[6][q] = F.By; sF[7][q] = F.Bz; }
     }
     __syncthreads();
     double vmax = 0.0;
+    const f64::Widths wd{};  // 1D grids do not divide their CFL speed by dx
     for (int q = threadIdx.x; q < TS; q += blockDim.x) {   // cell p = p0 + q
         const int p = p0 + q;
         if (p < np) {
             Prim<double> w0 = getw(q + 2);
             Prim<double> nw = w0;
+            double speed = 0.0;
+            bool bad = false;
             auto fget = [&](int qq) {
                 Cons<double> c;
                 c.rho = sF[0][qq]; c.E = sF[1][qq]; c.mx = sF[2][qq]; c.my = sF[3][qq]; c.mz = sF[4][qq];
@@ -378,14 +379,18 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
             };
             if (p >= 1 && p <= np - 2) {
                 Cons<double> fl = fget(q), fr = fget(q + 1);
-                nw = to_prim<MHD>(c_add<MHD>(to_cons<MHD>(w0), c_mul<MHD>(c_sub<MHD>(fl, fr), dt_dx)));
+                const f64::Updated r = f64::updated<MHD>(w0, sa, wd, c_mul<MHD>(c_sub<MHD>(fl, fr), dt_dx));
+                nw = r.w;
+                speed = r.speed;
+                bad = !is_physical<MHD>(nw);
+                // the last face's cell makes a second round trip (g >= 2: never a cell of the interior)
                 if (p == np - 2)
                     nw = to_prim<MHD>(c_add<MHD>(to_cons<MHD>(nw), c_mul<MHD>(c_sub<MHD>(fr, fr), dt_dx)));
             }
             const int c = p - G.g;
             if (c >= 0 && c < G.n[0]) {
-                if (!is_physical<MHD>(nw)) record_error(ctl, ST_UNPHYSICAL, p);
-                vmax = speed_max(vmax, cfl_speed_1d<MHD>(nw));
+                if (bad) record_error(ctl, ST_UNPHYSICAL, p);
+                vmax = speed_max(vmax, speed);
             }
             store_prim<MHD>(wout, PL, p, nw);
         }

@@ -23,6 +23,7 @@
 #include "recon.cuh"
 #include "riemann.cuh"
 #include "scratch.h"
+#include "solve64.cuh"
 
 namespace dgpu {
 
@@ -114,6 +115,65 @@ __device__ __forceinline__ Prim<double> body_field(Prim<double> w, double bx, do
     return w;
 }
 
+namespace f64 {
+
+// A cell after its flux differences with its field replaced by the faces':
+// its state, whether its conservative state was finite, and (SPEED) whether
+// the state is physical and its CFL speed.
+struct MhdCell {
+    Prim<double> w;
+    bool finite, physical;
+    double speed;
+};
+struct MhdField {
+    double bx, by, bz;
+};
+template <bool SPEED>
+__device__ __noinline__ void mhd_cell_plain(MhdCell* o, const Cons<double>* dU, int nd, const MhdField* b,
+                                            const StepArgs* sa) {
+    Cons<double> U = dgpu::to_cons<true>(o->w);
+    for (int k = 0; k < nd; k++) U = c_add<true>(U, dU[k]);
+    o->finite = is_finite<true>(U);
+    o->w = dgpu::body_field(dgpu::to_prim<true>(U), b->bx, b->by, b->bz, sa->ct_energy);
+    if (SPEED) {
+        o->physical = is_physical<true>(o->w);
+        o->speed = dgpu::cfl_speed<true>(o->w, sa->cfl, sa->dx, sa->dy, nd > 2 ? sa->dz : 0.0);
+    }
+}
+template <bool SPEED, class... D>
+__device__ __forceinline__ MhdCell mhd_cell(const Prim<double>& w, const StepArgs& sa, const MhdField& b, const D&... d) {
+    Chk ck;
+    ck.pos(w.p);
+    Cons<double> U = f64::to_cons<true>(w);
+    ((U = c_add<true>(U, d)), ...);
+    const Rec r = rec(U.rho, ck);
+    ck.fin(U.E);
+    ck.fin(U.Bx);
+    ck.fin(U.By);
+    ck.fin(U.Bz);
+    MhdCell o;
+    o.finite = o.physical = true;
+    o.w = f64::body_field(f64::to_prim<true>(U, r, ck), b.bx, b.by, b.bz, sa.ct_energy, r, ck);
+    o.speed = 0.0;
+    if (SPEED) {
+        sound_state<true>(o.w, ck);
+        o.speed = f64::cfl_speed(o.w, f64::fast_speed_max(o.w, r, ck), sa.cfl,
+                                 f64::widths(sizeof...(D), sa.dx, sa.dy, sa.dz), ck);
+    }
+    if (ck.bad) {
+        const Cons<double> all[] = {d...};
+        const StepArgs s = sa;
+        const MhdField f = b;
+        MhdCell t;
+        t.w = w;
+        mhd_cell_plain<SPEED>(&t, all, sizeof...(D), &f, &s);
+        o = t;
+    }
+    return o;
+}
+
+}  // namespace f64
+
 struct Mhd2DArgs {
     Geo G, FG;
     const double* w;     // cell state in
@@ -169,7 +229,7 @@ __device__ __forceinline__ void mhd2d_halfstates(const Mhd2DArgs& A, const Tile2
     const long long m = gidx2(F, i, j);
     int fo = 0;
     Prim<double> L, R;
-    fo += !muscl<true>(A.sa.limiter, W(i - 1, j), L, wc, R, W(i + 1, j), dt_dx, dBx, dBy, 0.0);
+    fo += !f64::muscl<true>(A.sa.limiter, W(i - 1, j), L, wc, R, W(i + 1, j), dt_dx, dBx, dBy, 0.0);
     L.Bx = bx0;
     R.Bx = bx1;
     store_prim<true>(A.S.hs, SP, m, L);
@@ -177,7 +237,7 @@ __device__ __forceinline__ void mhd2d_halfstates(const Mhd2DArgs& A, const Tile2
     Prim<double> yl = W(i, j - 1), yc = wc, yr = W(i, j + 1);
     swap_xy(yl); swap_xy(yc); swap_xy(yr);
     // swapped source terms: dB.y from the x faces, dB.x from the y faces
-    fo += !muscl<true>(A.sa.limiter, yl, L, yc, R, yr, dt_dy, dBy, dBx, 0.0);
+    fo += !f64::muscl<true>(A.sa.limiter, yl, L, yc, R, yr, dt_dy, dBy, dBx, 0.0);
     swap_xy(L); swap_xy(R);
     L.By = by0;
     R.By = by1;
@@ -205,13 +265,13 @@ __device__ __forceinline__ void mhd2d_prelim(const Mhd2DArgs& A, const Tile2& T)
     if (i >= -1 && i <= nx + 1 && j <= ny + 1) {
         Prim<double> L = load_prim<true>(A.S.hs + 8 * SP, SP, gidx2(F, i - 1, j));
         Prim<double> R = load_prim<true>(A.S.hs, SP, gidx2(F, i, j));
-        face_flux<true, SOLVER, 0>(L, R, dt_dx, eo, Fl, &st);
+        f64::face_flux<true, SOLVER, 0>(L, R, dt_dx, eo, Fl, &st);
         store_cons8(A.S.fx, SP, gidx2(F, i, j), Fl);
     }
     if (i <= nx + 1 && j >= -1 && j <= ny + 1) {
         Prim<double> L = load_prim<true>(A.S.hs + 24 * SP, SP, gidx2(F, i, j - 1));
         Prim<double> R = load_prim<true>(A.S.hs + 16 * SP, SP, gidx2(F, i, j));
-        face_flux<true, SOLVER, 1>(L, R, dt_dy, eo, Fl, &st);
+        f64::face_flux<true, SOLVER, 1>(L, R, dt_dy, eo, Fl, &st);
         store_cons8(A.S.fy, SP, gidx2(F, i, j), Fl);
     }
     warp_add_stat(&A.ctl->hlld_to_hlle, st.hlld_to_hlle);
@@ -279,13 +339,11 @@ __device__ __forceinline__ void mhd2d_half(const Mhd2DArgs& A, const Tile2& T) {
     const Cons<double> px0 = load_cons8(A.S.fx, SP, m), px1 = load_cons8(A.S.fx, SP, gidx2(F, i + 1, j));
     const Cons<double> py0 = load_cons8(A.S.fy, SP, m), py1 = load_cons8(A.S.fy, SP, gidx2(F, i, j + 1));
     {
-        Cons<double> U = to_cons<true>(W);
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(px0, px1), hdx));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(py0, py1), hdy));
-        if (!is_finite<true>(U)) record_error(A.ctl, ST_NAN, m);
-        Prim<double> wh = to_prim<true>(U);
-        wh = body_field(wh, (bxh0 + bxh1) * 0.5, (byh0 + byh1) * 0.5, bzh, A.sa.ct_energy);
-        store_v3(A.S.eh, SP, m, body_e(wh));
+        const f64::MhdCell h = f64::mhd_cell<false>(W, A.sa, f64::MhdField{(bxh0 + bxh1) * 0.5, (byh0 + byh1) * 0.5, bzh},
+                                                    c_mul<true>(c_sub<true>(px0, px1), hdx),
+                                                    c_mul<true>(c_sub<true>(py0, py1), hdy));
+        if (!h.finite) record_error(A.ctl, ST_NAN, m);
+        store_v3(A.S.eh, SP, m, body_e(h.w));
     }
     // CTU corrections (CTU.cpp:163-201)
     const double dBx = (A.B[gidx2(F, i + 1, j)] - A.B[gidx2(F, i, j)]) * dt_dx;
@@ -296,12 +354,8 @@ __device__ __forceinline__ void mhd2d_half(const Mhd2DArgs& A, const Tile2& T) {
         const double lim_z = lim_minmod(-dBy, dBx);
         corr.E += k1_8pi * (W.Bz * W.vz * lim_z);
         corr.Bz = 0.5 * dt_dy * (e01.x - e00.x) + 0.5 * W.vz * lim_z;
-        Cons<double> uL = c_add<true>(to_cons<true>(load_prim<true>(A.S.hs, SP, m)), corr);
-        Cons<double> uR = c_add<true>(to_cons<true>(load_prim<true>(A.S.hs + 8 * SP, SP, m)), corr);
-        uL.Bx = bxh0;
-        uR.Bx = bxh1;
-        store_prim<true>(A.S.hs, SP, m, to_prim<true>(uL));
-        store_prim<true>(A.S.hs + 8 * SP, SP, m, to_prim<true>(uR));
+        store_prim<true>(A.S.hs, SP, m, f64::corrected_mhd<0>(load_prim<true>(A.S.hs, SP, m), corr, bxh0));
+        store_prim<true>(A.S.hs + 8 * SP, SP, m, f64::corrected_mhd<0>(load_prim<true>(A.S.hs + 8 * SP, SP, m), corr, bxh1));
     }
     {
         Cons<double> corr = c_mul<true>(c_mul<true>(c_sub<true>(px0, px1), 0.5), dt_dx);
@@ -309,12 +363,8 @@ __device__ __forceinline__ void mhd2d_half(const Mhd2DArgs& A, const Tile2& T) {
         const double lim_z = lim_minmod(-dBx, dBy);
         corr.E += k1_8pi * (W.Bz * W.vz * lim_z);
         corr.Bz = -0.5 * dt_dx * (e10.y - e00.y) + 0.5 * W.vz * lim_z;
-        Cons<double> uL = c_add<true>(to_cons<true>(load_prim<true>(A.S.hs + 16 * SP, SP, m)), corr);
-        Cons<double> uR = c_add<true>(to_cons<true>(load_prim<true>(A.S.hs + 24 * SP, SP, m)), corr);
-        uL.By = byh0;
-        uR.By = byh1;
-        store_prim<true>(A.S.hs + 16 * SP, SP, m, to_prim<true>(uL));
-        store_prim<true>(A.S.hs + 24 * SP, SP, m, to_prim<true>(uR));
+        store_prim<true>(A.S.hs + 16 * SP, SP, m, f64::corrected_mhd<1>(load_prim<true>(A.S.hs + 16 * SP, SP, m), corr, byh0));
+        store_prim<true>(A.S.hs + 24 * SP, SP, m, f64::corrected_mhd<1>(load_prim<true>(A.S.hs + 24 * SP, SP, m), corr, byh1));
     }
 }
 
@@ -335,13 +385,13 @@ __device__ __forceinline__ void mhd2d_final_flux(const Mhd2DArgs& A, const Tile2
     if (i >= 0) {
         Prim<double> L = load_prim<true>(A.S.hs + 8 * SP, SP, gidx2(F, i - 1, j));
         Prim<double> R = load_prim<true>(A.S.hs, SP, gidx2(F, i, j));
-        face_flux<true, SOLVER, 0>(L, R, dt_dx, eo, Fl, &st);
+        f64::face_flux<true, SOLVER, 0>(L, R, dt_dx, eo, Fl, &st);
         store_cons8(A.S.fx, SP, gidx2(F, i, j), Fl);
     }
     if (j >= 0) {
         Prim<double> L = load_prim<true>(A.S.hs + 24 * SP, SP, gidx2(F, i, j - 1));
         Prim<double> R = load_prim<true>(A.S.hs + 16 * SP, SP, gidx2(F, i, j));
-        face_flux<true, SOLVER, 1>(L, R, dt_dy, eo, Fl, &st);
+        f64::face_flux<true, SOLVER, 1>(L, R, dt_dy, eo, Fl, &st);
         store_cons8(A.S.fy, SP, gidx2(F, i, j), Fl);
     }
     warp_add_stat(&A.ctl->hlld_to_hlle, st.hlld_to_hlle);
@@ -380,21 +430,19 @@ __device__ __forceinline__ void mhd2d_update(const Mhd2DArgs& A, const Tile2& T)
         const double by1 = A.B[FP + gidx2(F, i, j + 1)] - -(e11.z - e01.z) * dt_dx;
         const double bz = A.B[2 * FP + gidx2(F, i, j)] - ((e10.y - e00.y) * dt_dx - (e01.x - e00.x) * dt_dy);
         const long long mc = gidx2(G, i, j), mf = gidx2(F, i, j);
-        Cons<double> U = to_cons<true>(load_prim<true>(A.w, P, mc));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(load_cons8(A.S.fx, SP, mf),
-                                                   load_cons8(A.S.fx, SP, gidx2(F, i + 1, j))), dt_dx));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(load_cons8(A.S.fy, SP, mf),
-                                                   load_cons8(A.S.fy, SP, gidx2(F, i, j + 1))), dt_dy));
-        if (!is_finite<true>(U)) record_error(A.ctl, ST_NAN, mc);
-        Prim<double> nw = body_field(to_prim<true>(U), (bx0 + bx1) * 0.5, (by0 + by1) * 0.5, bz, A.sa.ct_energy);
-        if (!is_physical<true>(nw)) record_error(A.ctl, ST_UNPHYSICAL, mc);
-        store_prim<true>(A.wout, P, mc, nw);
+        const f64::MhdCell c = f64::mhd_cell<true>(
+            load_prim<true>(A.w, P, mc), A.sa, f64::MhdField{(bx0 + bx1) * 0.5, (by0 + by1) * 0.5, bz},
+            c_mul<true>(c_sub<true>(load_cons8(A.S.fx, SP, mf), load_cons8(A.S.fx, SP, gidx2(F, i + 1, j))), dt_dx),
+            c_mul<true>(c_sub<true>(load_cons8(A.S.fy, SP, mf), load_cons8(A.S.fy, SP, gidx2(F, i, j + 1))), dt_dy));
+        if (!c.finite) record_error(A.ctl, ST_NAN, mc);
+        if (!c.physical) record_error(A.ctl, ST_UNPHYSICAL, mc);
+        store_prim<true>(A.wout, P, mc, c.w);
         A.Bout[mf] = bx0;
         A.Bout[FP + mf] = by0;
         A.Bout[2 * FP + mf] = bz;
         if (i == nx - 1) A.Bout[gidx2(F, nx, j)] = bx1;
         if (j == ny - 1) A.Bout[FP + gidx2(F, i, ny)] = by1;
-        vmax = cfl_speed<true>(nw, A.sa.cfl, A.sa.dx, A.sa.dy, 0.0);
+        vmax = c.speed;
     }
     // block-wide max over a 2D block
     for (int o = 16; o > 0; o >>= 1) vmax = speed_max(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));

@@ -90,7 +90,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_halfstates(Mhd3DArgs A) {
     int fo = 0;
     Prim<double> L, R;
     // x (computeHalfStates_X 3D, Unsplit.cpp:351-378)
-    fo += !muscl<true>(A.sa.limiter, W(i - 1, j, k), L, wc, R, W(i + 1, j, k), dt_dx, dBx, dBy, dBz);
+    fo += !f64::muscl<true>(A.sa.limiter, W(i - 1, j, k), L, wc, R, W(i + 1, j, k), dt_dx, dBx, dBy, dBz);
     L.Bx = bx0;
     R.Bx = bx1;
     store_prim<true>(m3_hs(A, 0, 0), SP, f, L);
@@ -99,7 +99,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_halfstates(Mhd3DArgs A) {
     {
         Prim<double> a = W(i, j - 1, k), c = wc, b = W(i, j + 1, k);
         swap_xy(a); swap_xy(c); swap_xy(b);
-        fo += !muscl<true>(A.sa.limiter, a, L, c, R, b, dt_dy, dBy, dBx, dBz);
+        fo += !f64::muscl<true>(A.sa.limiter, a, L, c, R, b, dt_dy, dBy, dBx, dBz);
         swap_xy(L); swap_xy(R);
         L.By = by0;
         R.By = by1;
@@ -110,7 +110,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_halfstates(Mhd3DArgs A) {
     {
         Prim<double> a = W(i, j, k - 1), c = wc, b = W(i, j, k + 1);
         swap_xz(a); swap_xz(c); swap_xz(b);
-        fo += !muscl<true>(A.sa.limiter, a, L, c, R, b, dt_dz, dBz, dBy, dBx);
+        fo += !f64::muscl<true>(A.sa.limiter, a, L, c, R, b, dt_dz, dBz, dBy, dBx);
         swap_xz(L); swap_xz(R);
         L.Bz = bz0;
         R.Bz = bz1;
@@ -129,7 +129,7 @@ __device__ __forceinline__ void m3_face_flux(const Mhd3DArgs& A, int i, int j, i
     const Prim<double> L = m3_ld_prim(m3_hs(A, AX, 1), SP, gidx3(F, i - di, j - dj, k - dk));
     const Prim<double> R = m3_ld_prim(m3_hs(A, AX, 0), SP, gidx3(F, i, j, k));
     Cons<double> Fl;
-    face_flux<true, SOLVER, AX>(L, R, dtn, exact_opts(A.sa), Fl, st);
+    f64::face_flux<true, SOLVER, AX>(L, R, dtn, exact_opts(A.sa), Fl, st);
     store_cons8(m3_flux_w(A, AX), SP, gidx3(F, i, j, k), Fl);
 }
 
@@ -215,6 +215,11 @@ __device__ __forceinline__ M3Faces m3_faraday(const Mhd3DArgs& A, int i, int j, 
     return M3Faces{bx(i), bx(i + 1), by(j), by(j + 1), bz(k), bz(k + 1)};
 }
 
+template <int AX>
+struct M3Axis {
+    static constexpr int value = AX;
+};
+
 // K4
 static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
     __shared__ int s;
@@ -235,30 +240,24 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
     const Cons<double> pz0 = m3_ld_cons(A.S.fz, SP, m), pz1 = m3_ld_cons(A.S.fz, SP, gidx3(F, i, j, k + 1));
     {
         // applyFluxes g=1 at dt/2 (Unsplit.cpp:272-288), computeBodyFields, bodyElectric
-        Cons<double> U = to_cons<true>(W);
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(px0, px1), hdx));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(py0, py1), hdy));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(pz0, pz1), hdz));
-        if (!is_finite<true>(U)) record_error(A.ctl, ST_NAN, m);
-        Prim<double> wh = to_prim<true>(U);
-        wh = body_field(wh, (h.bx0 + h.bx1) * 0.5, (h.by0 + h.by1) * 0.5, (h.bz0 + h.bz1) * 0.5, A.sa.ct_energy);
-        store_v3(A.S.eh, SP, m, body_e(wh));
+        const f64::MhdCell c = f64::mhd_cell<false>(
+            W, A.sa, f64::MhdField{(h.bx0 + h.bx1) * 0.5, (h.by0 + h.by1) * 0.5, (h.bz0 + h.bz1) * 0.5},
+            c_mul<true>(c_sub<true>(px0, px1), hdx), c_mul<true>(c_sub<true>(py0, py1), hdy),
+            c_mul<true>(c_sub<true>(pz0, pz1), hdz));
+        if (!c.finite) record_error(A.ctl, ST_NAN, m);
+        store_v3(A.S.eh, SP, m, body_e(c.w));
     }
     // CTU corrections (CTU.cpp:66-129)
     const double dBx = (m3_ld(A.B, gidx3(F, i + 1, j, k)) - m3_ld(A.B, m)) * dt_dx;
     const double dBy = (m3_ld(A.B, FP + gidx3(F, i, j + 1, k)) - m3_ld(A.B, FP + m)) * dt_dy;
     const double dBz = (m3_ld(A.B, 2 * FP + gidx3(F, i, j, k + 1)) - m3_ld(A.B, 2 * FP + m)) * dt_dz;
     auto E0 = [&](int a, int b, int c) { return m3_ld_v3(A.S.e0, SP, gidx3(F, a, b, c)); };
-    auto apply = [&](int axis, Cons<double> corr, double bl, double br) {
-        double* pl = m3_hs(A, axis, 0);
-        double* pr = m3_hs(A, axis, 1);
-        Cons<double> uL = c_add<true>(to_cons<true>(load_prim<true>(pl, SP, m)), corr);
-        Cons<double> uR = c_add<true>(to_cons<true>(load_prim<true>(pr, SP, m)), corr);
-        if (axis == 0) { uL.Bx = bl; uR.Bx = br; }
-        else if (axis == 1) { uL.By = bl; uR.By = br; }
-        else { uL.Bz = bl; uR.Bz = br; }
-        store_prim<true>(pl, SP, m, to_prim<true>(uL));
-        store_prim<true>(pr, SP, m, to_prim<true>(uR));
+    auto apply = [&](auto axis, const Cons<double>& corr, double bl, double br) {
+        constexpr int AX = decltype(axis)::value;
+        double* pl = m3_hs(A, AX, 0);
+        double* pr = m3_hs(A, AX, 1);
+        store_prim<true>(pl, SP, m, f64::corrected_mhd<AX>(load_prim<true>(pl, SP, m), corr, bl));
+        store_prim<true>(pr, SP, m, f64::corrected_mhd<AX>(load_prim<true>(pr, SP, m), corr, br));
     };
     {   // x states
         Cons<double> corr = c_mul<true>(c_add<true>(c_mul<true>(c_sub<true>(py0, py1), dt_dy),
@@ -270,7 +269,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
                   0.5 * W.vy * lim_y;
         corr.Bz = 0.25 * dt_dy * (E0(i, j + 1, k).x - E0(i, j, k).x + E0(i, j + 1, k + 1).x - E0(i, j, k + 1).x) +
                   0.5 * W.vz * lim_z;
-        apply(0, corr, h.bx0, h.bx1);
+        apply(M3Axis<0>{}, corr, h.bx0, h.bx1);
     }
     {   // y states
         Cons<double> corr = c_mul<true>(c_add<true>(c_mul<true>(c_sub<true>(px0, px1), dt_dx),
@@ -282,7 +281,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
                   0.5 * W.vx * lim_x;
         corr.Bz = -0.25 * dt_dx * (E0(i + 1, j, k).y - E0(i, j, k).y + E0(i + 1, j, k + 1).y - E0(i, j, k + 1).y) +
                   0.5 * W.vz * lim_z;
-        apply(1, corr, h.by0, h.by1);
+        apply(M3Axis<1>{}, corr, h.by0, h.by1);
     }
     {   // z states
         Cons<double> corr = c_mul<true>(c_add<true>(c_mul<true>(c_sub<true>(px0, px1), dt_dx),
@@ -294,7 +293,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
                   0.5 * W.vx * lim_x;
         corr.By = 0.25 * dt_dx * (E0(i + 1, j, k).z - E0(i, j, k).z + E0(i + 1, j + 1, k).z - E0(i, j + 1, k).z) +
                   0.5 * W.vy * lim_y;
-        apply(2, corr, h.bz0, h.bz1);
+        apply(M3Axis<2>{}, corr, h.bz0, h.bz1);
     }
 }
 
@@ -315,22 +314,22 @@ static __global__ void k_m3_update(Mhd3DArgs A) {
         const int nx = G.n[0], ny = G.n[1], nz = G.n[2];
         const long long mc = gidx3(G, i, j, k), mf = gidx3(F, i, j, k);
         const M3Faces b = m3_faraday(A, i, j, k, dt_dx, dt_dy, dt_dz);
-        Cons<double> U = to_cons<true>(m3_ld_prim(A.w, P, mc));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fx, SP, mf), m3_ld_cons(A.S.fx, SP, gidx3(F, i + 1, j, k))), dt_dx));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fy, SP, mf), m3_ld_cons(A.S.fy, SP, gidx3(F, i, j + 1, k))), dt_dy));
-        U = c_add<true>(U, c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fz, SP, mf), m3_ld_cons(A.S.fz, SP, gidx3(F, i, j, k + 1))), dt_dz));
-        if (!is_finite<true>(U)) record_error(A.ctl, ST_NAN, mc);
-        Prim<double> nw = body_field(to_prim<true>(U), (b.bx0 + b.bx1) * 0.5, (b.by0 + b.by1) * 0.5, (b.bz0 + b.bz1) * 0.5,
-                                     A.sa.ct_energy);
-        if (!is_physical<true>(nw)) record_error(A.ctl, ST_UNPHYSICAL, mc);
-        store_prim<true>(A.wout, P, mc, nw);
+        const f64::MhdCell c = f64::mhd_cell<true>(
+            m3_ld_prim(A.w, P, mc), A.sa,
+            f64::MhdField{(b.bx0 + b.bx1) * 0.5, (b.by0 + b.by1) * 0.5, (b.bz0 + b.bz1) * 0.5},
+            c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fx, SP, mf), m3_ld_cons(A.S.fx, SP, gidx3(F, i + 1, j, k))), dt_dx),
+            c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fy, SP, mf), m3_ld_cons(A.S.fy, SP, gidx3(F, i, j + 1, k))), dt_dy),
+            c_mul<true>(c_sub<true>(m3_ld_cons(A.S.fz, SP, mf), m3_ld_cons(A.S.fz, SP, gidx3(F, i, j, k + 1))), dt_dz));
+        if (!c.finite) record_error(A.ctl, ST_NAN, mc);
+        if (!c.physical) record_error(A.ctl, ST_UNPHYSICAL, mc);
+        store_prim<true>(A.wout, P, mc, c.w);
         A.Bout[mf] = b.bx0;
         A.Bout[FP + mf] = b.by0;
         A.Bout[2 * FP + mf] = b.bz0;
         if (i == nx - 1) A.Bout[gidx3(F, nx, j, k)] = b.bx1;
         if (j == ny - 1) A.Bout[FP + gidx3(F, i, ny, k)] = b.by1;
         if (k == nz - 1) A.Bout[2 * FP + gidx3(F, i, j, nz)] = b.bz1;
-        vmax = cfl_speed<true>(nw, A.sa.cfl, A.sa.dx, A.sa.dy, A.sa.dz);
+        vmax = c.speed;
     }
     vmax = block_max(vmax, red);
     if (threadIdx.x == 0) atomic_max_speed(&A.ctl->vmax[A.sa.slot_out], vmax);

@@ -13,6 +13,7 @@
 #include "grid.cuh"
 #include "recon.cuh"
 #include "riemann.cuh"
+#include "solve64.cuh"
 
 namespace dgpu {
 
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(256) k_sweep(Geo G, const double* __restrict__
         const int p = p0 - 1 + c;
         if (L0 + l < nlines && p >= 1 && p <= np - 2) {
             Prim<double> oL, oR;
-            muscl<false>(sa.limiter, W_at(l, c), oL, W_at(l, c + 1), oR, W_at(l, c + 2), dt_dx, 0.0, 0.0, 0.0);
+            f64::muscl<false>(sa.limiter, W_at(l, c), oL, W_at(l, c + 1), oR, W_at(l, c + 2), dt_dx, 0.0, 0.0, 0.0);
             put_hs(sL, l, c, oL);
             put_hs(sR, l, c, oR);
         }
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(256) k_sweep(Geo G, const double* __restrict__
         const Prim<double> Lf = (p == 0) ? W_at(l, c + 1) : get_hs(sR, l, c);
         const Prim<double> Rf = (p + 1 == np - 1) ? W_at(l, c + 2) : get_hs(sL, l, c + 1);
         Cons<double> F;
-        if (!face_flux_x<false, SOLVER>(Lf, Rf, dt_dx, eo, F, &st)) record_error(ctl, ST_FINAL_FLUX, sweep_elem<DIM, AX>(G, L, p));
+        if (!f64::face_flux_x<false, SOLVER>(Lf, Rf, dt_dx, eo, F, &st)) record_error(ctl, ST_FINAL_FLUX, sweep_elem<DIM, AX>(G, L, p));
         sF[(0 * TL + l) * (TC + 1) + c] = F.rho;
         sF[(1 * TL + l) * (TC + 1) + c] = F.E;
         sF[(2 * TL + l) * (TC + 1) + c] = F.mx;
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(256) k_sweep(Geo G, const double* __restrict__
         Prim<double> nw = W_at(l, c + 2);
         if (p >= 1 && p <= np - 2) {
             const Cons<double> fl = fget(l, c), fr = fget(l, c + 1);
-            nw = to_prim<false>(c_add<false>(to_cons<false>(nw), c_mul<false>(c_sub<false>(fl, fr), dt_dx)));
+            nw = f64::corrected<false>(nw, c_mul<false>(c_sub<false>(fr, fl), dt_dx));
             if (p == np - 2) nw = to_prim<false>(c_add<false>(to_cons<false>(nw), c_mul<false>(c_sub<false>(fr, fr), dt_dx)));
         }
         swap_axis<AX>(nw);
