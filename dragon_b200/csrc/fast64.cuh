@@ -51,12 +51,16 @@ namespace f64 {
 // to zero. A quotient that is a velocity, a field or a flux component raises
 // the flag when its numerator is smaller (quots); one that is only added to
 // something of normal size, which it then cannot change, passes as it is
-// (quotn). Dividing the small ones on the spot instead of raising the flag
-// was 1 % faster on the 3D blast, whose ambient gas is full of them, and 8 %
-// slower on the shear layer (a branch per group of quotients).
+// (quotn).
 
-// The flag of one face, cell or state.
-struct Chk {
+// The flag of one face, cell or state. With LOCAL the quotients of small
+// numerators are divided by the plain operator on the spot: a branch per group
+// of quotients (the shear layer 8 % slower), which the gas ahead of a 3D blast
+// repays (its step 7 % faster). Elsewhere a raised flag first repeats the work
+// out of line with LOCAL, and with the plain operators if that raises it too.
+template <bool LOCAL>
+struct Flag {
+    static constexpr bool kLocal = LOCAL;
     bool bad = false;
     // |x| in [2^-120, 2^50)
     __device__ __forceinline__ void den(double x) {
@@ -79,6 +83,15 @@ struct Chk {
     }
     __device__ __forceinline__ void raise(bool c) { bad |= c; }
 };
+using Chk = Flag<false>;
+
+// 0 < |x| < 2^-920
+__device__ __forceinline__ bool tiny(double x) {
+    const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return u < ((1023u - 920u) << 20) && (u | (unsigned)__double2loint(x)) != 0u;
+}
+static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+
 // 1 / b, rounded. The corrections round down the one case whose exact value
 // lies just above a rounding boundary, a significand of all ones: 2^k for 2^k
 // (1 + 2^-52).
@@ -102,7 +115,8 @@ __device__ __forceinline__ Rec rec_of(double b) {
     const double y = reciprocal(b);
     return Rec{b, y, __dmul_rn(y, __fma_rn(-b, y, 1.0))};
 }
-__device__ __forceinline__ Rec rec(double b, Chk& ck) {
+template <class C>
+__device__ __forceinline__ Rec rec(double b, C& ck) {
     ck.den(b);
     return rec_of(b);
 }
@@ -122,15 +136,27 @@ __device__ __forceinline__ double quot(double a, const Rec& r) {
     return signed_as(q, a, r.b);
 }
 // a / r.b of a value that a small quotient cannot change.
-__device__ __forceinline__ double quotn(double a, const Rec& r, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double quotn(double a, const Rec& r, C& ck) {
     ck.fin(a);
     return quot(a, r);
 }
 // a / r.b for several values at once.
-template <class... D>
-__device__ __forceinline__ void quots(const Rec& r, Chk& ck, D&... a) {
-    (ck.num(a), ...);
-    ((a = quot(a, r)), ...);
+template <class C, class... D>
+__device__ __forceinline__ void quots(const Rec& r, C& ck, D&... a) {
+    if constexpr (C::kLocal) {
+        (ck.fin(a), ...);
+        const bool small = (tiny(a) || ...);
+        const double n[sizeof...(D)] = {a...};
+        ((a = quot(a, r)), ...);
+        if (small) {
+            int k = 0;
+            ((a = div_plain(n[k++], r.b)), ...);
+        }
+    } else {
+        (ck.num(a), ...);
+        ((a = quot(a, r)), ...);
+    }
 }
 // a / b, one quotient (the first correction takes the place of the second
 // part of the reciprocal), without a look at the ranges
@@ -141,7 +167,8 @@ __device__ __forceinline__ double div_of(double a, double b) {
     q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return signed_as(q, a, b);
 }
-__device__ __forceinline__ double div(double a, double b, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double div(double a, double b, C& ck) {
     ck.num(a);
     ck.den(b);
     return div_of(a, b);
@@ -158,12 +185,14 @@ __device__ __forceinline__ double root_of(double a) {
     return __fma_rn(__fma_rn(-g, g, a), h, g);
 }
 // sqrt(a), a > 0 in range
-__device__ __forceinline__ double root(double a, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double root(double a, C& ck) {
     ck.raise((unsigned)__double2hiint(a) - ((1023u - 900u) << 20) >= (1800u << 20));
     return root_of(a);
 }
 // sqrt(a), a >= 0 of a value that a root below 2^-450 cannot change (0 then)
-__device__ __forceinline__ double root0(double a, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double root0(double a, C& ck) {
     const unsigned u = (unsigned)__double2hiint(a);
     const bool z = u < ((1023u - 900u) << 20) || (u == 0x80000000u && __double2loint(a) == 0);
     ck.raise(!z && u >= ((1023u + 900u) << 20));
@@ -207,15 +236,15 @@ __device__ __forceinline__ Cons<double> to_cons(const Prim<double>& w) {
 }
 // a / (2 b) is half of a / b: a quotient near the smallest normal number, where
 // it would not be, does not change E
-template <bool MHD>
-__device__ __forceinline__ double pressure(const Cons<double>& u, const Rec& r, Chk& ck) {
+template <bool MHD, class C>
+__device__ __forceinline__ double pressure(const Cons<double>& u, const Rec& r, C& ck) {
     ck.pos(u.E);
     double Eth = u.E - 0.5 * quotn(dot3(u.mx, u.my, u.mz, u.mx, u.my, u.mz), r, ck);
     if constexpr (MHD) Eth -= dot3(u.Bx, u.By, u.Bz, u.Bx, u.By, u.Bz) * k1_8pi;
     return kGm1 * Eth;
 }
-template <bool MHD>
-__device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const Rec& r, Chk& ck) {
+template <bool MHD, class C>
+__device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const Rec& r, C& ck) {
     Prim<double> w;
     w.rho = u.rho;
     w.vx = u.mx;
@@ -229,8 +258,8 @@ __device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const Rec
 }
 // The flag unless is_physical holds for a state that to_prim gave without
 // one (its velocities are finite then).
-template <bool MHD>
-__device__ __forceinline__ void sound_state(const Prim<double>& w, Chk& ck) {
+template <bool MHD, class C>
+__device__ __forceinline__ void sound_state(const Prim<double>& w, C& ck) {
     ck.pos(w.rho);
     ck.pos(w.p);
     if constexpr (MHD) {
@@ -245,9 +274,9 @@ __device__ __noinline__ void corrected_plain(Prim<double>* w, const Cons<double>
     *w = dgpu::to_prim<MHD>(dgpu::c_sub<MHD>(dgpu::to_cons<MHD>(*w), *d));
 }
 // to_prim(to_cons(w) - d): a half state with its transverse correction.
-template <bool MHD>
+template <bool MHD, bool LOCAL = false>
 __device__ __forceinline__ Prim<double> corrected(const Prim<double>& w, const Cons<double>& d) {
-    Chk ck;
+    Flag<LOCAL> ck;
     ck.pos(w.p);
     const Cons<double> u = c_sub<MHD>(f64::to_cons<MHD>(w), d);
     Prim<double> r = f64::to_prim<MHD>(u, rec(u.rho, ck), ck);
@@ -278,7 +307,8 @@ __device__ __forceinline__ Widths widths(int dim, double dx, double dy, double d
 }
 // cfl_speed of a cell with sound (or fast) speed a, for the sum and the
 // maximum over the axes; the p-norm raises the flag.
-__device__ __forceinline__ double cfl_speed(const Prim<double>& w, double a, int cfl, const Widths& d, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double cfl_speed(const Prim<double>& w, double a, int cfl, const Widths& d, C& ck) {
     ck.raise(d.bad || cfl > 1);
     double s = quotn(fabs(w.vx) + a, d.x, ck);
     const double t = quotn(fabs(w.vy) + a, d.y, ck);
@@ -319,11 +349,13 @@ __device__ __forceinline__ Cons<double> flux_of(const Cons<double>& u, double p,
 }
 
 // Wave speeds (fluid.cuh), r the reciprocal of the density.
-__device__ __forceinline__ double sound_speed(const Prim<double>& w, const Rec& r, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double sound_speed(const Prim<double>& w, const Rec& r, C& ck) {
     ck.pos(w.p);
     return root(quot(kGamma * w.p, r), ck);
 }
-__device__ __forceinline__ double fast_speed(const Prim<double>& w, double Bk, const Rec& r, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double fast_speed(const Prim<double>& w, double Bk, const Rec& r, C& ck) {
     const double c = f64::sound_speed(w, r, ck);
     const double a = by_sq4pi(root0(quotn(dot3(w.Bx, w.By, w.Bz, w.Bx, w.By, w.Bz), r, ck), ck));
     const double c2 = c * c, a2 = a * a, ak2 = quotn(Bk * Bk, r, ck) * k1_4pi;
@@ -331,7 +363,8 @@ __device__ __forceinline__ double fast_speed(const Prim<double>& w, double Bk, c
     const double disc = smax(0.0, (s * s) * 0.25 - ak2 * c2);
     return root((c2 + a2) * 0.5 + root0(disc, ck), ck);
 }
-__device__ __forceinline__ double fast_speed_max(const Prim<double>& w, const Rec& r, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double fast_speed_max(const Prim<double>& w, const Rec& r, C& ck) {
     double Bk;
     if (w.Bx * w.Bx < w.By * w.By) Bk = (w.Bx * w.Bx < w.Bz * w.Bz) ? w.Bx : w.Bz;
     else Bk = (w.By * w.By < w.Bz * w.Bz) ? w.By : w.Bz;
@@ -342,8 +375,8 @@ __device__ __forceinline__ double fast_speed_max(const Prim<double>& w, const Re
 // pressure test E - m^2 / (2 rho) - B^2 / (8 pi) > 0, rounded as the plain
 // test rounds it, follows from the inequality without a division where it
 // holds with a margin of 2^-44 E; the states between go to the plain test.
-template <bool MHD>
-__device__ __forceinline__ void surely_physical(const Cons<double>& u, Chk& ck) {
+template <bool MHD, class C>
+__device__ __forceinline__ void surely_physical(const Cons<double>& u, C& ck) {
     const double m2 = dot3(u.mx, u.my, u.mz, u.mx, u.my, u.mz);
     ck.pos(u.rho);
     ck.pos(u.E);

@@ -3,7 +3,7 @@
 // face_flux() bit for bit. Each first computes without a branch per division
 // and raises a flag on anything out of the ordinary (an operand out of range,
 // an unphysical or borderline state, a fallback of the solver); the face or
-// cell is then repeated by the plain routine, out of line.
+// cell is then repeated out of line, in the end by the plain routine.
 #pragma once
 
 #include "fast64.cuh"
@@ -15,13 +15,20 @@ namespace f64 {
 
 // n / d for slopes of one sign (on), 0 otherwise. With n at least 2^-900 the
 // divisor may be smaller than elsewhere.
-__device__ __forceinline__ double slope_quot(double n, double d, bool on, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double slope_quot(double n, double d, bool on, C& ck) {
     const unsigned un = (unsigned)__double2hiint(n) & 0x7fffffffu, ud = (unsigned)__double2hiint(d) & 0x7fffffffu;
-    ck.raise(on && (un - ((1023u - 900u) << 20) >= (1800u << 20) || ud - ((1023u - 450u) << 20) >= (500u << 20)));
+    const bool odd = on && (un - ((1023u - 900u) << 20) >= (1800u << 20) || ud - ((1023u - 450u) << 20) >= (500u << 20));
+    if constexpr (C::kLocal) {
+        if (odd) return div_plain(n, d);
+    } else {
+        ck.raise(odd);
+    }
     const double q = div_of(n, on ? d : 1.0);
     return on ? q : 0.0;
 }
-__device__ __forceinline__ double limit1(int lim, double a, double b, Chk& ck) {
+template <class C>
+__device__ __forceinline__ double limit1(int lim, double a, double b, C& ck) {
     switch (lim) {
         case LIM_MC: return lim_mc(a, b);
         // the plain form divides (2 a) b by a + b unless a b <= 0
@@ -33,10 +40,10 @@ __device__ __forceinline__ double limit1(int lim, double a, double b, Chk& ck) {
 }
 
 // TVD::MUSCL with both predicted states physical (else the flag).
-template <bool MHD>
+template <bool MHD, class C>
 __device__ __forceinline__ void muscl_body(int lim, const Prim<double>& wL, Prim<double>& outL, const Prim<double>& wC,
                                            Prim<double>& outR, const Prim<double>& wR, double dt_dL, double dBx,
-                                           double dBy, double dBz, Chk& ck) {
+                                           double dBy, double dBz, C& ck) {
     Prim<double> dW, L, Rr;
     dW.rho = f64::limit1(lim, wC.rho - wL.rho, wR.rho - wC.rho, ck);
     dW.vx = f64::limit1(lim, wC.vx - wL.vx, wR.vx - wC.vx, ck);
@@ -88,22 +95,31 @@ __device__ __forceinline__ void muscl_body(int lim, const Prim<double>& wL, Prim
     sound_state<MHD>(outR, ck);
 }
 
-template <bool MHD>
-__device__ __noinline__ bool muscl_plain(int lim, const Prim<double>* w3, Prim<double>* out2, double dt_dL, double dBx,
-                                         double dBy, double dBz) {
-    return dgpu::muscl<MHD>(lim, w3[0], out2[0], w3[1], out2[1], w3[2], dt_dL, dBx, dBy, dBz);
+// Out of line, for a cell whose flag is up: with small numerators divided on
+// the spot (AGAIN), else with the plain operators.
+template <bool MHD, bool AGAIN>
+__device__ __noinline__ bool muscl_slow(int lim, const Prim<double>* w3, Prim<double>* out2, double dt_dL, double dBx,
+                                        double dBy, double dBz) {
+    if constexpr (AGAIN) {
+        Flag<true> ck;
+        muscl_body<MHD>(lim, w3[0], out2[0], w3[1], out2[1], w3[2], dt_dL, dBx, dBy, dBz, ck);
+        if (!ck.bad) return true;
+        return muscl_slow<MHD, false>(lim, w3, out2, dt_dL, dBx, dBy, dBz);
+    } else {
+        return dgpu::muscl<MHD>(lim, w3[0], out2[0], w3[1], out2[1], w3[2], dt_dL, dBx, dBy, dBz);
+    }
 }
 
-template <bool MHD>
+template <bool MHD, bool LOCAL = false>
 __device__ __forceinline__ bool muscl(int lim, const Prim<double>& wL, Prim<double>& outL, const Prim<double>& wC,
                                       Prim<double>& outR, const Prim<double>& wR, double dt_dL, double dBx, double dBy,
                                       double dBz) {
-    Chk ck;
+    Flag<LOCAL> ck;
     muscl_body<MHD>(lim, wL, outL, wC, outR, wR, dt_dL, dBx, dBy, dBz, ck);
     if (!ck.bad) return true;
     const Prim<double> w3[3] = {wL, wC, wR};
     Prim<double> out2[2];
-    const bool ok = muscl_plain<MHD>(lim, w3, out2, dt_dL, dBx, dBy, dBz);
+    const bool ok = muscl_slow<MHD, !LOCAL>(lim, w3, out2, dt_dL, dBx, dBy, dBz);
     outL = out2[0];
     outR = out2[1];
     return ok;
@@ -117,7 +133,8 @@ struct FaceSide {
     Cons<double> U;
     double a, sq, h;  // sound speed, sqrt(rho), enthalpy
 };
-__device__ __forceinline__ void face_side(const Prim<double>& w, FaceSide& s, Chk& ck) {
+template <class C>
+__device__ __forceinline__ void face_side(const Prim<double>& w, FaceSide& s, C& ck) {
     ck.pos(w.p);
     s.r = rec(w.rho, ck);
     s.U = f64::to_cons<false>(w);
@@ -125,8 +142,9 @@ __device__ __forceinline__ void face_side(const Prim<double>& w, FaceSide& s, Ch
     s.sq = root(w.rho, ck);
 }
 // Roe-averaged normal velocity and sound speed (HLL::roeAvg)
+template <class C>
 __device__ __forceinline__ void roe_mean(const Prim<double>& L, const Prim<double>& Rt, const FaceSide& sL,
-                                         const FaceSide& sR, double& vx, double& aM, Chk& ck) {
+                                         const FaceSide& sR, double& vx, double& aM, C& ck) {
     const Rec rs = rec(sL.sq + sR.sq, ck);
     const double _sql = quot(sL.sq, rs), _sqr = quot(sR.sq, rs);
     const double rho = sL.sq * sR.sq;
@@ -140,14 +158,16 @@ __device__ __forceinline__ void roe_mean(const Prim<double>& L, const Prim<doubl
     aM = root(div(kGamma * by_gamma(ar), rho, ck), ck);
 }
 // x-flux of one side's state
-__device__ __forceinline__ Cons<double> side_flux(const Prim<double>& w, const FaceSide& s, Chk& ck) {
+template <class C>
+__device__ __forceinline__ Cons<double> side_flux(const Prim<double>& w, const FaceSide& s, C& ck) {
     return flux_of<false>(s.U, f64::pressure<false>(s.U, s.r, ck), w.vx, w.vy, w.vz);
 }
 
 // Riemann::HLLC: one path for the supersonic and the star cases, the flux of
 // the upwind side plus the star part.
+template <class C>
 __device__ __forceinline__ Cons<double> hllc(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
-                                             Chk& ck) {
+                                             C& ck) {
     face_side(L, sL, ck);
     face_side(Rt, sR, ck);
     double vM, aM;
@@ -183,8 +203,9 @@ __device__ __forceinline__ Cons<double> hllc(const Prim<double>& L, const Prim<d
 }
 
 // Riemann::HLL(SL, SR)
+template <class C>
 __device__ __forceinline__ Cons<double> hll_speeds(const Prim<double>& L, const Prim<double>& Rt, const FaceSide& sL,
-                                                   const FaceSide& sR, double sl, double sr, Chk& ck) {
+                                                   const FaceSide& sR, double sl, double sr, C& ck) {
     const Cons<double> FL = side_flux(L, sL, ck), FR = side_flux(Rt, sR, ck);
     if (sl >= 0.0) return FL;
     if (sr <= 0.0) return FR;
@@ -194,16 +215,18 @@ __device__ __forceinline__ Cons<double> hll_speeds(const Prim<double>& L, const 
     quots(rec(sr - sl, ck), ck, F.rho, F.E, F.mx, F.my, F.mz);
     return F;
 }
+template <class C>
 __device__ __forceinline__ Cons<double> hll(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
-                                            Chk& ck) {
+                                            C& ck) {
     face_side(L, sL, ck);
     face_side(Rt, sR, ck);
     double vM, aM;
     roe_mean(L, Rt, sL, sR, vM, aM, ck);
     return hll_speeds(L, Rt, sL, sR, smin(L.vx - sL.a, vM - aM), smax(Rt.vx + sR.a, vM + aM), ck);
 }
+template <class C>
 __device__ __forceinline__ Cons<double> hlle(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
-                                             Chk& ck) {
+                                             C& ck) {
     face_side(L, sL, ck);
     face_side(Rt, sR, ck);
     const double sql = sL.sq, sqr = sR.sq, aL = sL.a, aR = sR.a;
@@ -218,8 +241,9 @@ __device__ __forceinline__ Cons<double> hlle(const Prim<double>& L, const Prim<d
 
 // Riemann::Roe with the Harten-Hyman fix; the two entropy-fix returns raise
 // the flag (transonic rarefactions are few).
+template <class C>
 __device__ __forceinline__ Cons<double> roe(const Prim<double>& L, const Prim<double>& Rt, FaceSide& sL, FaceSide& sR,
-                                            Chk& ck) {
+                                            C& ck) {
     face_side(L, sL, ck);
     face_side(Rt, sR, ck);
     const Rec rs = rec(sL.sq + sR.sq, ck);
@@ -260,6 +284,132 @@ __device__ __forceinline__ Cons<double> roe(const Prim<double>& L, const Prim<do
 }
 
 // ---------------------------------------------------------------------------
+// The exact solver (Exact.cpp) with the reference's mean guess. What bounds it
+// is pow, so a power of one (a uniform or a resting gas, both sides of most
+// faces ahead of a front) is not taken, and the derivative's power -(g + 1) /
+// (2 g) is the function's (g - 1) / (2 g) divided by the argument (their sum
+// is -1): it steers the Newton step alone, whose end the tolerance sets.
+
+__device__ __forceinline__ double pow1(double x, double y) { return x == 1.0 ? 1.0 : pow(x, y); }
+
+struct ExactSide {
+    Rec rp;              // 1 / p
+    double a, A, B, ra;  // sound speed, Riemann::f's A and B, rho a
+};
+template <class C>
+__device__ __forceinline__ void exact_side(const Prim<double>& w, ExactSide& s, C& ck) {
+    const Rec r = rec(w.rho, ck);
+    ck.pos(w.rho);
+    ck.pos(w.p);
+    s.a = root(quot(kGamma * w.p, r), ck);
+    s.A = quot(k2_Gp1, r);
+    s.B = kGm1_Gp1 * w.p;
+    s.ra = w.rho * s.a;
+    s.rp = rec(w.p, ck);
+}
+template <bool DERIV, class C>
+__device__ __forceinline__ double exact_f(double p, const Prim<double>& w, const ExactSide& s, double& df, C& ck) {
+    if (p > w.p) {
+        const Rec r = rec(s.B + p, ck);
+        const double q = root(quot(s.A, r), ck), d = p - w.p;
+        if constexpr (DERIV) df = q * (1.0 - 0.5 * quotn(d, r, ck));
+        return d * q;
+    }
+    ck.pos(p);
+    const double x = quot(p, s.rp), y = pow1(x, kGm1_2G);
+    if constexpr (DERIV) df = div(y, x * s.ra, ck);
+    return k2_Gm1 * s.a * (y - 1.0);
+}
+template <class C>
+__device__ __forceinline__ double exact_rho(double p, const Prim<double>& w, const ExactSide& s, C& ck) {
+    if (p > w.p) return div(w.rho * (p + s.B), kGm1_Gp1 * p + w.p, ck);
+    return w.rho * pow1(quot(p, s.rp), kGinv);
+}
+// the flux of the exact solution at x / t = 0
+template <class C>
+__device__ __forceinline__ Cons<double> exact(const Prim<double>& L, const Prim<double>& Rt, const ExactOpts& o,
+                                              FaceStats* st, C& ck) {
+    ExactSide sL, sR;
+    exact_side(L, sL, ck);
+    exact_side(Rt, sR, ck);
+    double v, p, rhoL, rhoR, dfL = 0.0, dfR = 0.0;
+    const double p_min = smin(L.p, Rt.p);
+    if (exact_f<false>(p_min, L, sL, dfL, ck) + exact_f<false>(p_min, Rt, sR, dfR, ck) + Rt.vx - L.vx >= 0.0) {
+        st->trrs += 1;
+        const double _LR = div(pow1(quot(L.p, sR.rp), kGm1_2G) * sR.a, sL.a, ck);
+        v = div(_LR * L.vx + Rt.vx + k2_Gm1 * (_LR * sL.a - sR.a), _LR + 1.0, ck);
+        p = L.p * pow1(1.0 - div(kGm1_2 * (v - L.vx), sL.a, ck), k2G_Gm1);
+        ck.pos(p);
+        rhoL = L.rho * pow1(quot(p, sL.rp), kGinv);
+        rhoR = Rt.rho * pow1(quot(p, sR.rp), kGinv);
+    } else {
+        p = (L.p + Rt.p) * 0.5;
+        double CHA;
+        int iters = o.max_iters, n = 0;
+        do {
+            const double fL = exact_f<true>(p, L, sL, dfL, ck), fR = exact_f<true>(p, Rt, sR, dfR, ck);
+            double delta = fL + fR + Rt.vx - L.vx;
+            delta = smin(div(delta, dfL + dfR, ck), 0.8 * p);
+            p -= delta;
+            CHA = fabs(div(delta, p + delta * 0.5, ck));
+            n++;
+        } while (CHA > o.tol && --iters != 0 && !ck.bad);
+        st->newton_iters += n;
+        st->exact_calls += 1;
+        st->cap_hits += CHA > o.tol;
+        const double fR = exact_f<false>(p, Rt, sR, dfR, ck);
+        v = (L.vx + Rt.vx + fR - exact_f<false>(p, L, sL, dfL, ck)) * 0.5;
+        rhoL = exact_rho(p, L, sL, ck);
+        rhoR = exact_rho(p, Rt, sR, ck);
+    }
+    ck.pos(p);
+    ck.num(v);
+    Prim<double> w;
+    w.Bx = w.By = w.Bz = 0;
+    if (fabs(v - 0.0) < 1e-12) {
+        // on the contact: the root-density mean of both star states
+        const double sql = root(rhoL, ck), sqr = root(rhoR, ck);
+        const Prim<double> a{rhoL, p, v, L.vy, L.vz, 0, 0, 0}, b{rhoR, p, v, Rt.vy, Rt.vz, 0, 0, 0};
+        Cons<double> u = c_add<false>(c_mul<false>(f64::to_cons<false>(a), sql), c_mul<false>(f64::to_cons<false>(b), sqr));
+        quots(rec(sql + sqr, ck), ck, u.rho, u.E, u.mx, u.my, u.mz);
+        w = f64::to_prim<false>(u, rec(u.rho, ck), ck);
+    } else {
+        // the side the contact leaves behind, mirrored to be the right one
+        const bool left = 0.0 < v;
+        Prim<double> W = left ? L : Rt;
+        const double a = left ? sL.a : sR.a, rho = left ? rhoL : rhoR;
+        const Rec rp = left ? sL.rp : sR.rp;
+        if (left) W.vx *= -1.0;
+        const double sv = left ? v * -1.0 : v, x_t = left ? -0.0 : 0.0;
+        w = W;
+        int zone;
+        if (p > W.p) {
+            const double scale = root(quot(kGp1_2G * p, rp) + kGm1_2G, ck);
+            zone = (x_t - W.vx > scale * a) ? 1 : 3;
+        } else {
+            if (x_t - W.vx > a) zone = 1;
+            else if (x_t - sv > a) zone = 2;
+            else zone = (x_t - sv > a * pow1(quot(p, rp), kGm1_2G)) ? 2 : 3;
+        }
+        if (zone == 3) {
+            w.rho = rho;
+            w.p = p;
+            w.vx = sv;
+        } else if (zone == 2) {
+            const double scale = k2_Gp1 - div(kGm1_Gp1 * (W.vx - x_t), a, ck);
+            w.rho *= pow1(scale, k2_Gm1);
+            w.p *= pow1(scale, k2G_Gm1);
+            w.vx = k2_Gp1 * (x_t - a + W.vx * kGm1_2);
+        }
+        if (left) w.vx *= -1.0;
+    }
+    ck.pos(w.rho);
+    ck.pos(w.p);
+    const Cons<double> U = f64::to_cons<false>(w);
+    return flux_of<false>(U, f64::pressure<false>(U, rec(U.rho, ck), ck), w.vx, w.vy, w.vz);
+}
+
+// ---------------------------------------------------------------------------
 // MHD solvers. The normal field is averaged into both sides first, as the
 // plain routines do.
 
@@ -267,7 +417,8 @@ struct MhdSide {
     Rec r;        // of the density
     double E, c;  // energy, fast speed along x
 };
-__device__ __forceinline__ void mhd_side(const Prim<double>& w, MhdSide& s, Chk& ck) {
+template <class C>
+__device__ __forceinline__ void mhd_side(const Prim<double>& w, MhdSide& s, C& ck) {
     s.r = rec(w.rho, ck);
     s.c = f64::fast_speed(w, w.Bx, s.r, ck);
     s.E = f64::energy<true>(w);
@@ -275,7 +426,8 @@ __device__ __forceinline__ void mhd_side(const Prim<double>& w, MhdSide& s, Chk&
 __device__ __forceinline__ Cons<double> mhd_cons(const Prim<double>& w, const MhdSide& s) {
     return Cons<double>{w.rho, s.E, w.vx * w.rho, w.vy * w.rho, w.vz * w.rho, w.Bx, w.By, w.Bz};
 }
-__device__ __forceinline__ Cons<double> mhd_flux(const Prim<double>& w, const MhdSide& s, Chk& ck) {
+template <class C>
+__device__ __forceinline__ Cons<double> mhd_flux(const Prim<double>& w, const MhdSide& s, C& ck) {
     const Cons<double> U = mhd_cons(w, s);
     return flux_of<true>(U, f64::pressure<true>(U, s.r, ck), w.vx, w.vy, w.vz);
 }
@@ -288,9 +440,9 @@ struct MhdStar {
     Cons<double> u, F;
     Prim<double> w;
 };
-template <bool ZERO, bool FLUX>
+template <bool ZERO, bool FLUX, class C>
 __device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s, double x, double SK, double SM,
-                                         const Rec& d, double rho, double pT, double Bx, MhdStar& o, Chk& ck) {
+                                         const Rec& d, double rho, double pT, double Bx, MhdStar& o, C& ck) {
     Cons<double> u;
     u.rho = rho;
     double vy, vz;
@@ -351,7 +503,8 @@ __device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s
 // and energy (SsL >= 0 implies SM >= 0, SsR <= 0 implies SM <= 0), so the
 // other side's star state comes first and leaves its velocity and field:
 // fewer values alive at a time (both sides whole spilled 700 bytes).
-__device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, Chk& ck) {
+template <class C>
+__device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, C& ck) {
     const double Bx = (L.Bx + Rt.Bx) * 0.5;
     L.Bx = Bx;
     Rt.Bx = Bx;
@@ -431,7 +584,8 @@ __device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, Ch
 }
 
 // Riemann::HLLE for MHD states
-__device__ __forceinline__ Cons<double> hlle_mhd(Prim<double> L, Prim<double> Rt, Chk& ck) {
+template <class C>
+__device__ __forceinline__ Cons<double> hlle_mhd(Prim<double> L, Prim<double> Rt, C& ck) {
     const double Bx = (L.Bx + Rt.Bx) * 0.5;
     L.Bx = Bx;
     Rt.Bx = Bx;
@@ -455,53 +609,83 @@ __device__ __forceinline__ Cons<double> hlle_mhd(Prim<double> L, Prim<double> Rt
     return F;
 }
 
-template <bool MHD, int SOLVER>
-__device__ __noinline__ bool face_plain(const Prim<double>* LR, double dt_dx, const ExactOpts* eo, Cons<double>* F,
-                                        FaceStats* st) {
-    return face_flux_x<MHD, SOLVER, double>(LR[0], LR[1], dt_dx, *eo, *F, st);
+// The solver and the physicality test of its flux (verify_and_fallback,
+// Flux.cpp:77-97); a test that fails or is close raises the flag.
+template <bool MHD, int SOLVER, class C>
+__device__ __forceinline__ void face_body(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
+                                          const ExactOpts& eo, Cons<double>& F, FaceStats* st, C& ck) {
+    if constexpr (MHD) {
+        if constexpr (SOLVER == RS_HLLE) F = hlle_mhd(L, Rt, ck);
+        else F = hlld(L, Rt, ck);
+    } else {
+        FaceSide sL, sR;
+        if constexpr (SOLVER == RS_HLL) F = hll(L, Rt, sL, sR, ck);
+        else if constexpr (SOLVER == RS_HLLE) F = hlle(L, Rt, sL, sR, ck);
+        else if constexpr (SOLVER == RS_ROE) F = roe(L, Rt, sL, sR, ck);
+        else if constexpr (SOLVER == RS_EXACT) {
+            F = exact(L, Rt, eo, st, ck);
+            sL.U = f64::to_cons<false>(L);
+            sR.U = f64::to_cons<false>(Rt);
+        } else F = hllc(L, Rt, sL, sR, ck);
+        if (dt_dL > 0.0) {
+            surely_physical<false>(c_sub<false>(sL.U, c_mul<false>(F, dt_dL)), ck);
+            surely_physical<false>(c_add<false>(sR.U, c_mul<false>(F, dt_dL)), ck);
+        }
+    }
+}
+template <bool MHD, int SOLVER, bool AGAIN>
+__device__ __noinline__ bool face_slow(const Prim<double>* LR, double dt_dx, const ExactOpts* eo, Cons<double>* F,
+                                       FaceStats* st) {
+    if constexpr (AGAIN) {
+        Flag<true> ck;
+        FaceStats s = *st;
+        face_body<MHD, SOLVER>(LR[0], LR[1], dt_dx, *eo, *F, &s, ck);
+        if (!ck.bad) {
+            *st = s;
+            return true;
+        }
+        return face_slow<MHD, SOLVER, false>(LR, dt_dx, eo, F, st);
+    } else {
+        return face_flux_x<MHD, SOLVER, double>(LR[0], LR[1], dt_dx, *eo, *F, st);
+    }
 }
 
-// The flux along x of the states on both sides of a face, as face_flux_x. The
-// exact solver is pow and MHD HLL is rare: they take the plain routine.
-template <bool MHD, int SOLVER>
+// The flux along x of the states on both sides of a face, as face_flux_x. MHD
+// HLL is rare and takes the plain routine, and so does the exact solver with
+// another guess than the mean or while its solves are logged.
+template <bool MHD, int SOLVER, bool LOCAL = false>
 __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
                                             const ExactOpts& eo, Cons<double>& F, FaceStats* st) {
-    if constexpr (MHD ? SOLVER == RS_HLL : SOLVER == RS_EXACT) {
+    if constexpr (MHD && SOLVER == RS_HLL) {
         return dgpu::face_flux_x<MHD, SOLVER>(L, Rt, dt_dL, eo, F, st);
     } else {
-        Chk ck;
-        if constexpr (MHD) {
-            if constexpr (SOLVER == RS_HLLE) F = hlle_mhd(L, Rt, ck);
-            else F = hlld(L, Rt, ck);
-        } else {
-            FaceSide sL, sR;
-            if constexpr (SOLVER == RS_HLL) F = hll(L, Rt, sL, sR, ck);
-            else if constexpr (SOLVER == RS_HLLE) F = hlle(L, Rt, sL, sR, ck);
-            else if constexpr (SOLVER == RS_ROE) F = roe(L, Rt, sL, sR, ck);
-            else F = hllc(L, Rt, sL, sR, ck);
-            // verify_and_fallback (Flux.cpp:77-97)
-            if (dt_dL > 0.0) {
-                surely_physical<false>(c_sub<false>(sL.U, c_mul<false>(F, dt_dL)), ck);
-                surely_physical<false>(c_add<false>(sR.U, c_mul<false>(F, dt_dL)), ck);
+        constexpr bool kExact = !MHD && SOLVER == RS_EXACT;
+        Flag<LOCAL> ck;
+        FaceStats s = *st;
+        const bool plain = kExact && (eo.guess != GUESS_MEAN || eo.log.rows);
+        if (!plain) {
+            face_body<MHD, SOLVER>(L, Rt, dt_dL, eo, F, &s, ck);
+            if (!ck.bad) {
+                if constexpr (kExact) *st = s;
+                return true;
             }
         }
-        if (!ck.bad) return true;
         const Prim<double> LR[2] = {L, Rt};
         Cons<double> G;
         const ExactOpts e = eo;
-        FaceStats s = *st;
-        const bool ok = face_plain<MHD, SOLVER>(LR, dt_dL, &e, &G, &s);
-        *st = s;
+        FaceStats t = *st;
+        const bool ok = face_slow<MHD, SOLVER, !LOCAL && !kExact>(LR, dt_dL, &e, &G, &t);
+        *st = t;
         F = G;
         return ok;
     }
 }
-template <bool MHD, int SOLVER, int AX>
+template <bool MHD, int SOLVER, int AX, bool LOCAL = false>
 __device__ __forceinline__ bool face_flux(Prim<double> L, Prim<double> Rt, double dt_dL, const ExactOpts& eo,
                                           Cons<double>& F, FaceStats* st) {
     swap_axis<AX>(L);
     swap_axis<AX>(Rt);
-    const bool ok = f64::face_flux_x<MHD, SOLVER>(L, Rt, dt_dL, eo, F, st);
+    const bool ok = f64::face_flux_x<MHD, SOLVER, LOCAL>(L, Rt, dt_dL, eo, F, st);
     swap_axis<AX>(F);
     return ok;
 }
@@ -511,7 +695,8 @@ __device__ __forceinline__ bool face_flux(Prim<double> L, Prim<double> Rt, doubl
 
 // protect_thermal's gate 8 pi p / B^2 <= 0.1 without the division, the flag
 // where the rounded quotient could fall on either side.
-__device__ __forceinline__ bool keeps_thermal(const Prim<double>& w, int mode, Chk& ck) {
+template <class C>
+__device__ __forceinline__ bool keeps_thermal(const Prim<double>& w, int mode, C& ck) {
     if (mode == 0) return false;
     if (mode == 1) return true;
     const double B2 = b2_of(w);
@@ -523,8 +708,9 @@ __device__ __forceinline__ bool keeps_thermal(const Prim<double>& w, int mode, C
 }
 // computeBodyField (B_fields.cpp:70-79): the cell with its field replaced, r
 // the reciprocal of its density.
+template <class C>
 __device__ __forceinline__ Prim<double> body_field(Prim<double> w, double bx, double by, double bz, int mode,
-                                                   const Rec& r, Chk& ck) {
+                                                   const Rec& r, C& ck) {
     const bool keep = keeps_thermal(w, mode, ck);
     ck.pos(w.p);
     Cons<double> U = f64::to_cons<true>(w);

@@ -90,7 +90,7 @@ static __global__ void k_h3_halfstates(Step3DArgs A) {
         Prim<double> c = wc, L, R;
         if (ax == 1) { swap_xy(wl); swap_xy(c); swap_xy(wr); }
         if (ax == 2) { swap_xz(wl); swap_xz(c); swap_xz(wr); }
-        fo += !f64::muscl<false>(A.sa.limiter, wl, L, c, R, wr, dts[ax], 0.0, 0.0, 0.0);
+        fo += !f64::muscl<false, true>(A.sa.limiter, wl, L, c, R, wr, dts[ax], 0.0, 0.0, 0.0);
         if (ax == 1) { swap_xy(L); swap_xy(R); }
         if (ax == 2) { swap_xz(L); swap_xz(R); }
         st5(A.S.hs + (10 * ax) * A.S.plane, A.S.plane, m, L);
@@ -110,7 +110,7 @@ __device__ __forceinline__ void h3_flux(const Step3DArgs& A, double* out, int i,
     Prim<double> R = ld5(A.S.hs + (10 * AX) * SP, SP, m);
     Cons<double> F;
     const ExactOpts eo = exact_opts(A.sa);
-    if (!f64::face_flux<false, SOLVER, AX>(L, R, dtn, eo, F, st)) record_error(A.ctl, stage, m);
+    if (!f64::face_flux<false, SOLVER, AX, true>(L, R, dtn, eo, F, st)) record_error(A.ctl, stage, m);
     stc5(out, SP, m, F);
 }
 
@@ -129,7 +129,7 @@ __device__ __forceinline__ Prim<double> h3_corrected_once(const Step3DArgs& A, c
     const long long SP = A.S.plane;
     const Cons<double> tr = c_mul<false>(
         c_sub<false>(ldc5(F, SP, gidx3(G, i + (D == 0), j + (D == 1), k + (D == 2))), ldc5(F, SP, gidx3(G, i, j, k))), w);
-    return f64::corrected<false>(s, tr);
+    return f64::corrected<false, true>(s, tr);
 }
 
 // The corrected half state of cell (i,j,k) along AX (SIDE 0: the state at the
@@ -165,7 +165,7 @@ __device__ __forceinline__ void h3_final_flux(const Step3DArgs& A, const H3Half&
     const Prim<double> L = h3_corrected<AX, 1>(A, h, i - di, j - dj, k - dk);
     const Prim<double> R = h3_corrected<AX, 0>(A, h, i, j, k);
     Cons<double> F;
-    if (!f64::face_flux<false, SOLVER, AX>(L, R, dtn, exact_opts(A.sa), F, st)) record_error(A.ctl, ST_FINAL_FLUX, m);
+    if (!f64::face_flux<false, SOLVER, AX, true>(L, R, dtn, exact_opts(A.sa), F, st)) record_error(A.ctl, ST_FINAL_FLUX, m);
     stc5(A.S.pf + 5 * AX * SP, SP, m, F);
 }
 
@@ -241,9 +241,9 @@ __device__ __forceinline__ void h3_ctu_flux_learned(const Step3DArgs& A, const d
             return c_mul<false>(c_sub<false>(t1, t0), dtT);
         };
         m = gidx3(G, i, j, k);
-        L = f64::corrected<false>(ld5(A.S.hs + (10 * AX + 5) * SP, SP, gidx3(G, i - di, j - dj, k - dk)),
+        L = f64::corrected<false, true>(ld5(A.S.hs + (10 * AX + 5) * SP, SP, gidx3(G, i - di, j - dj, k - dk)),
                                   trans(i - di, j - dj, k - dk));
-        R = f64::corrected<false>(ld5(A.S.hs + (10 * AX) * SP, SP, m), trans(i, j, k));
+        R = f64::corrected<false, true>(ld5(A.S.hs + (10 * AX) * SP, SP, m), trans(i, j, k));
     }
     const LearnedGuess<double> g = learned_guess_face<AX>(A, L, R, valid);
     if (!valid) return;
@@ -363,13 +363,13 @@ __device__ __forceinline__ void h3_ctu_flux(const Step3DArgs& A, const double* T
         const Cons<double> t1 = ldc5(T, SP, gidx3(G, a + ti, b + tj, c + tk)), t0 = ldc5(T, SP, gidx3(G, a, b, c));
         return c_mul<false>(c_sub<false>(t1, t0), dtT);
     };
-    const Prim<double> L = f64::corrected<false>(ld5(A.S.hs + (10 * AX + 5) * SP, SP, gidx3(G, i - di, j - dj, k - dk)),
+    const Prim<double> L = f64::corrected<false, true>(ld5(A.S.hs + (10 * AX + 5) * SP, SP, gidx3(G, i - di, j - dj, k - dk)),
                                                  trans(i - di, j - dj, k - dk));
     const long long m = gidx3(G, i, j, k);
-    const Prim<double> R = f64::corrected<false>(ld5(A.S.hs + (10 * AX) * SP, SP, m), trans(i, j, k));
+    const Prim<double> R = f64::corrected<false, true>(ld5(A.S.hs + (10 * AX) * SP, SP, m), trans(i, j, k));
     Cons<double> F;
     const ExactOpts eo = exact_opts(A.sa);
-    if (!f64::face_flux<false, SOLVER, AX>(L, R, dtn, eo, F, st)) record_error(A.ctl, ST_PRELIM_FLUX, m);
+    if (!f64::face_flux<false, SOLVER, AX, true>(L, R, dtn, eo, F, st)) record_error(A.ctl, ST_PRELIM_FLUX, m);
     stc5(out, SP, m, F);
 }
 

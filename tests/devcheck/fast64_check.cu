@@ -153,6 +153,7 @@ int f64_face(int mhd, int solver, long long n, const double* L, const double* R,
     } else if (solver == RS_HLL) k_face<false, RS_HLL><<<g, 128>>>(n, A.p, B.p, dt_dx, O.p);
     else if (solver == RS_HLLE) k_face<false, RS_HLLE><<<g, 128>>>(n, A.p, B.p, dt_dx, O.p);
     else if (solver == RS_ROE) k_face<false, RS_ROE><<<g, 128>>>(n, A.p, B.p, dt_dx, O.p);
+    else if (solver == RS_EXACT) k_face<false, RS_EXACT><<<g, 128>>>(n, A.p, B.p, dt_dx, O.p);
     else k_face<false, RS_HLLC><<<g, 128>>>(n, A.p, B.p, dt_dx, O.p);
     return done(O, out, 20 * n);
 }

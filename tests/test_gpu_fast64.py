@@ -177,6 +177,31 @@ def test_faces_bits(lib, mhd, solver):
         assert ok.all(), (L[~ok.all(1)][:3], R[~ok.all(1)][:3], out[:, ~ok.all(1)][:, :3])
 
 
+def test_exact_solver_faces(lib):
+    """The exact solver's Newton derivative takes one power where the plain form
+    takes two, so its star pressure may differ in the last places: a flux to
+    1e-13 of its largest component (the solve stops at a relative change of
+    1e-12, after which the quadratic convergence leaves rounding error), and the
+    same fallback decisions, on pairs of physical states a step apart."""
+    rng = np.random.default_rng(2)
+    L = states(rng, N, False)
+    R = neighbour(rng, L)
+    good = np.isfinite(L).all(1) & np.isfinite(R).all(1) & (L[:, :2] > 1e-3).all(1) & (R[:, :2] > 1e-3).all(1)
+    good &= (np.abs(L[:, 2:]) < 10).all(1) & (np.abs(R[:, 2:]) < 10).all(1)
+    L, R = np.ascontiguousarray(L[good]), np.ascontiguousarray(R[good])
+    n = len(L)
+    assert n > N // 3
+    out = np.zeros((2, n, 10))
+    assert lib.f64_face(0, 0, n, p(L), p(R), 0.05, p(out)) == 0
+    done = (out[0, :, 8] == 1) & (out[1, :, 8] == 1)
+    assert (out[0, :, 8:] == out[1, :, 8:]).all()
+    scale = np.abs(out[1, done, :8]).max(1, keepdims=True)
+    # six iterations cap the reference's Newton: a solve the cap ended is as far on either side
+    err = np.abs(out[0, done, :8] - out[1, done, :8]) / scale
+    assert np.quantile(err.max(1), 0.99) < 1e-13
+    assert err.max() < 1e-9
+
+
 @pytest.mark.parametrize("mhd", [0, 1])
 @pytest.mark.parametrize("limiter", range(5))
 def test_half_states_bits(lib, mhd, limiter):
