@@ -491,6 +491,253 @@ __global__ void __launch_bounds__(256) k_prologue_coop(Geo G, Geo FG, double* __
     if (lead) prologue_set_dt(G, ctl, pa, __longlong_as_double((long long)*(volatile unsigned long long*)&ctl->ring_bits));
 }
 
+// ---------------------------------------------------------------------------
+// The prologue of a 2D / 3D grid in one pass, without a grid barrier: every
+// ghost value is worked out from the cells no pass writes. A ghost cell walks
+// the list backwards: the last pass that writes it says which cell it copied,
+// that cell's last earlier writer says the next, until no pass is left; the
+// copied value then takes the passes' changes of sign, gates or fixed state.
+// With corner ghosts on, a pass along an axis writes every cell beyond its
+// face, so the walk ends in a cell that none writes (its coordinate along an
+// axis either became interior or lies where no pass writes), and all ghosts
+// can be filled at once. The ring's CFL speed comes from the values just
+// made, and the last CTA to finish does the bookkeeping and the dt.
+//
+// The cooperative kernel above needs a grid barrier after each axis and two
+// for the ring, and reads the ring again. Per launch, in a run of steps: shear
+// layer 1024^2 @@KH@@, 3D blast 128^3 @@B3@@, Orszag-Tang 384^2 @@OT@@. It stays for
+// lists with corner ghosts off, with Reflective or Fixed faces of an MHD grid
+// (their face-B passes read what they wrote) and for extents below the ghost
+// width.
+constexpr int kDirectEntries = 8;
+struct DirectList {
+    int n;
+    BCEntry e[kDirectEntries];
+};
+
+// Whether the entries [first, first + count) of a list can be filled in one pass.
+inline bool direct_fill_ok(const Geo& G, const BCEntry* e, int first, int count, bool mhd) {
+    if (G.dim < 2 || count > kDirectEntries) return false;
+    for (int a = 0; a < G.dim; a++)
+        if (G.n[a] < G.g + 1) return false;
+    for (int k = first; k < first + count; k++) {
+        if (e[k].type == BC_IGNORE) continue;
+        if (!e[k].corners) return false;
+        if (mhd && (e[k].type == BC_REFLECTIVE || e[k].type == BC_FIXED)) return false;
+    }
+    return true;
+}
+
+// Item t of the points of a padded box outside its interior [0, n): lo layers
+// below and hi above along every axis. False past the last.
+struct ShellBox {
+    int n[3], lo, hi, dim;
+    unsigned s0, s1, total;  // items of the first axis' slabs, of the first two
+};
+__host__ __device__ __forceinline__ ShellBox shell_box(const Geo& G, const int* n, int lo, int hi) {
+    ShellBox b;
+    b.dim = G.dim;
+    b.lo = lo;
+    b.hi = hi;
+    for (int a = 0; a < 3; a++) b.n[a] = a < G.dim ? n[a] : 1;
+    const unsigned w = lo + hi;
+    const unsigned e1 = G.dim > 1 ? n[1] + w : 1, e2 = G.dim > 2 ? n[2] + w : 1;
+    b.s0 = w * e1 * e2;
+    b.s1 = b.s0 + (unsigned)b.n[0] * w * e2;
+    b.total = G.dim > 2 ? b.s1 + (unsigned)b.n[0] * b.n[1] * w : b.s1;
+    return b;
+}
+__device__ __forceinline__ void shell_point(const ShellBox& b, unsigned t, int* c) {
+    const unsigned w = b.lo + b.hi;
+    const unsigned e1 = b.n[1] + w, e2 = b.dim > 2 ? b.n[2] + w : 1;
+    auto layer = [&](unsigned l, int n) { return (int)l < b.lo ? (int)l - b.lo : n + (int)l - b.lo; };
+    if (t < b.s0) {
+        const unsigned q = t / e2, k = t - q * e2;
+        c[0] = layer(q / e1, b.n[0]);
+        c[1] = (int)(q % e1) - b.lo;
+        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
+    } else if (t < b.s1) {
+        t -= b.s0;
+        const unsigned q = t / e2, k = t - q * e2;
+        c[0] = q / w;
+        c[1] = layer(q % w, b.n[1]);
+        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
+    } else {
+        t -= b.s1;
+        const unsigned q = t / w;
+        c[2] = layer(t - q * w, b.n[2]);
+        c[0] = q / b.n[1];
+        c[1] = q % b.n[1];
+    }
+}
+__device__ __forceinline__ long long gidx(const Geo& G, const int* c) {
+    return G.dim == 2 ? gidx2(G, c[0], c[1]) : gidx3(G, c[0], c[1], c[2]);
+}
+
+// The value of ghost cell c after every pass of the list; false if none writes it.
+template <bool MHD>
+__device__ __forceinline__ bool direct_cell(const Geo& G, const double* __restrict__ w, const DirectList& list,
+                                            const int* c, Prim<double>& v) {
+    int q[3] = {c[0], c[1], c[2]};
+    unsigned flip = 0, gate_lo = 0, gate_hi = 0;  // by axis
+    int fixed = -1;
+    bool hit = false;
+    for (int e = list.n - 1; e >= 0 && fixed < 0; e--) {
+        const int type = list.e[e].type, faces = list.e[e].faces;
+        if (type == BC_IGNORE) continue;
+#pragma unroll
+        for (int a = 2; a >= 0; a--) {
+            if (a >= G.dim || fixed >= 0) continue;
+            const int na = G.n[a], x = q[a];
+            const bool neg = x < 0;
+            if (!(neg || x >= na) || !(faces & (1 << (2 * a + (neg ? 0 : 1))))) continue;
+            hit = true;
+            if (type == BC_FIXED) {
+                fixed = e;
+            } else if (type == BC_PERIODIC) {
+                q[a] = neg ? x + na : x - na;
+            } else if (type == BC_REFLECTIVE) {
+                q[a] = neg ? -x - 1 : 2 * na - 1 - x;
+                flip |= 1u << a;
+            } else {
+                q[a] = neg ? 0 : na - 1;
+                if (type == BC_OUTFLOW_GATED) (neg ? gate_lo : gate_hi) |= 1u << a;
+            }
+        }
+    }
+    if (fixed >= 0) {
+        const double* s = list.e[fixed].state;
+        v = Prim<double>{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]};
+    } else {
+        v = load_prim<MHD>(w, G.plane, gidx(G, q));
+    }
+    // at most one pass per axis copied the value, and each changes its own
+    // axis' velocity (Reflective the field components too, by sign)
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        double& vel = a == 0 ? v.vx : a == 1 ? v.vy : v.vz;
+        if ((gate_lo >> a & 1) && vel > 0) vel = 0;
+        if ((gate_hi >> a & 1) && vel < 0) vel = 0;
+        if (flip >> a & 1) vel *= -1;
+    }
+    return hit;
+}
+
+// Component c of the face-centred B at point p (a point beyond the interior
+// faces) after every pass; false if none writes it. Outflow extrapolates the
+// normal component from the two faces next to it (bc_faces_axis).
+// Walks point q from pass `last` (3 entry + axis) down. Returns whether some
+// pass writes it; axis: the one an extrapolating pass stopped at (-1: none),
+// with the layers from the face and the pass to go on with.
+__device__ __forceinline__ bool direct_walk(const Geo& FG, const DirectList& list, const int* ncell, int comp, int last,
+                                            int* q, int& axis, int& steps, int& next) {
+    bool hit = false;
+    axis = -1;
+    for (int e = last / 3; e >= 0 && axis < 0; e--) {
+        const int type = list.e[e].type, faces = list.e[e].faces;
+        if (type == BC_IGNORE) continue;
+#pragma unroll
+        for (int a = 2; a >= 0; a--) {
+            if (a >= FG.dim || e * 3 + a > last || axis >= 0) continue;
+            const int na = ncell[a], x = q[a];
+            const bool neg = x < 0;
+            if (!(neg || x >= na) || !(faces & (1 << (2 * a + (neg ? 0 : 1))))) continue;
+            if (type == BC_PERIODIC) {
+                if (!neg && x - na >= FG.g) continue;  // the outermost point is not filled
+                q[a] = neg ? x + na : x - na;
+                hit = true;
+            } else if (a != comp) {
+                q[a] = neg ? 0 : na - 1;
+                hit = true;
+            } else if (neg || x > na) {
+                axis = a;
+                steps = neg ? -x : x - na;
+                q[a] = neg ? 0 : na;
+                next = e * 3 + a - 1;
+                hit = true;
+            }
+        }
+    }
+    return hit;
+}
+__device__ __forceinline__ bool direct_face(const Geo& FG, const double* __restrict__ B, const DirectList& list,
+                                            const int* ncell, const int* p, int comp, double& v) {
+    int q[3] = {p[0], p[1], p[2]}, axis, steps = 0, next = 0;
+    const double* Bc = B + comp * FG.plane;
+    if (!direct_walk(FG, list, ncell, comp, 3 * list.n - 1, q, axis, steps, next)) return false;
+    if (axis < 0) {
+        v = Bc[gidx(FG, q)];
+        return true;
+    }
+    // both supporting faces go on along the earlier passes (none extrapolates
+    // again: the component's own axis is done)
+    int r[3] = {q[0], q[1], q[2]}, ax, st, nx;
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        if (a == axis) r[a] += q[a] == 0 ? 1 : -1;
+    if (next >= 0) {
+        direct_walk(FG, list, ncell, comp, next, q, ax, st, nx);
+        direct_walk(FG, list, ncell, comp, next, r, ax, st, nx);
+    }
+    double b0 = Bc[gidx(FG, q)], b1 = Bc[gidx(FG, r)];
+    for (int s = 0; s < steps; s++) {
+        const double b = 2 * b0 - b1;
+        b1 = b0;
+        b0 = b;
+    }
+    v = b0;
+    return true;
+}
+
+template <bool MHD>
+__global__ void __launch_bounds__(128) k_prologue_direct(Geo G, Geo FG, double* __restrict__ w, double* __restrict__ B,
+                                                         const __grid_constant__ DirectList list, StepCtl* ctl,
+                                                         PrologueArgs pa, ShellBox cells, ShellBox faces) {
+    __shared__ int s_skip;
+    __shared__ double s_red[32];
+    if (threadIdx.x == 0) s_skip = *(const volatile int*)&ctl->err ? 1 : bookkeeping_done(ctl, pa) ? 2 : 0;
+    __syncthreads();
+    if (s_skip == 1) return;
+    if (s_skip == 0) {
+        double m = 0.0;
+        const unsigned nf = MHD && pa.apply_bc ? faces.total : 0;
+        const unsigned stride = gridDim.x * blockDim.x;
+        for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < cells.total + nf; t += stride) {
+            int c[3];
+            if (t < cells.total) {
+                shell_point(cells, t, c);
+                Prim<double> v;
+                if (direct_cell<MHD>(G, w, list, c, v)) store_prim<MHD>(w, G.plane, gidx(G, c), v);
+                bool ring = pa.compute_dt != 0;
+#pragma unroll
+                for (int a = 0; a < 3; a++) ring &= a >= G.dim || (c[a] >= -1 && c[a] <= G.n[a]);
+                if (ring) m = speed_max(m, cfl_speed<MHD>(v, pa.cfl, pa.dx, pa.dy, G.dim > 2 ? pa.dz : 0.0));
+            } else if constexpr (MHD) {
+                shell_point(faces, t - cells.total, c);
+                for (int k = 0; k < 3; k++) {
+                    double v;
+                    if (direct_face(FG, B, list, G.n, c, k, v)) B[k * FG.plane + gidx(FG, c)] = v;
+                }
+            }
+        }
+        if (pa.compute_dt) {
+            m = block_max(m, s_red);
+            if (threadIdx.x == 0) atomic_max_speed(&ctl->direct_ring, m);
+        }
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&ctl->direct_arrive, 1u) == gridDim.x - 1) {
+            __threadfence();
+            ctl->direct_arrive = 0u;
+            const double m = __longlong_as_double((long long)*(volatile unsigned long long*)&ctl->direct_ring);
+            ctl->direct_ring = 0ull;
+            const int over = prologue_bookkeeping(ctl, pa);
+            if (!over && pa.compute_dt) prologue_set_dt(G, ctl, pa, m);
+        }
+    }
+}
+
 // One ghost-fill pass (entry, axis; cells or faces) spread over a whole grid,
 // for grids whose ghost layers are too large for the one-CTA prologue. The
 // passes run as separate launches in the prologue's order (entry by entry,

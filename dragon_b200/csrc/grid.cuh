@@ -60,6 +60,9 @@ struct StepCtl {
     // ghost-ring max CFL speed (bits of a non-negative double)
     unsigned bar_arrive, bar_gen;
     unsigned long long ring_bits;
+    // the same of the one-pass prologue: arrivals and ring max, zero between launches
+    unsigned direct_arrive, pad1;
+    unsigned long long direct_ring;
     // interior max CFL speed (bits of a non-negative double): slots 0/1 ping-pong
     // with the state buffers, slot 2 is scratch for cfl_time. Kept last: the
     // host rewrites everything before it when a new advance starts.

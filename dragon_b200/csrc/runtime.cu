@@ -323,6 +323,24 @@ static int launch_prologue_range(dragon_grid* h, int c, int bookkeeping, int app
         else k_prologue<false><<<1, 1024, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
         h->launches++;
     };
+    // 2D / 3D: one pass over the ghost shell where the list allows it; with no
+    // entries it reads the ring alone (a cfl_time on the current ghosts)
+    if (h->dbg_stall_cta < 0 && !h->dbg_no_coop && (apply_bc || compute_dt) &&
+        direct_fill_ok(h->cg, h->hbcs.data(), bc_first, apply_bc ? bc_count : 0, h->mhd)) {
+        DirectList list{};
+        list.n = apply_bc ? bc_count : 0;
+        for (int k = 0; k < list.n; k++) list.e[k] = h->hbcs[bc_first + k];
+        const ShellBox cells = shell_box(h->cg, h->n, h->g, h->g), faces = shell_box(h->fg, h->n, h->g, h->g + 1);
+        const unsigned items = cells.total + (h->mhd && apply_bc ? faces.total : 0);
+        const int blocks = (int)std::min<unsigned>((items + 127) / 128, 148 * 16);
+        if (h->mhd)
+            k_prologue_direct<true><<<blocks, 128, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
+        else
+            k_prologue_direct<false><<<blocks, 128, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
+        CK(cudaGetLastError());
+        h->launches++;
+        return 0;
+    }
     if (h->dim == 1 || !apply_bc || bc_count == 0) {
         one_cta(pa);
         CK(cudaGetLastError());
