@@ -57,6 +57,25 @@ __global__ void k_batch_summary(const BatchInst* __restrict__ insts, int n, Summ
     out[i] = Summary{ldv(&c->err), ldv(&c->done), ldv(&c->steps_done), ldv(&c->cur)};
 }
 
+// The members' control blocks between their own memory and one array, so that
+// an advance moves them with one copy each way: SCATTER writes each member's
+// header (everything before vmax) from it, else it gathers whole blocks. A
+// copy and a wait per member each way was 1.1 ms of a 48-member advance.
+template <bool SCATTER>
+__global__ void k_batch_ctl(const BatchInst* __restrict__ insts, int n, StepCtl* __restrict__ all) {
+    static_assert(sizeof(StepCtl) % 8 == 0 && offsetof(StepCtl, vmax) % 8 == 0, "copied in words");
+    constexpr int W = (int)((SCATTER ? offsetof(StepCtl, vmax) : sizeof(StepCtl)) / 8);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n * 32) return;
+    const int i = t / 32;
+    unsigned long long* a = reinterpret_cast<unsigned long long*>(all + i);
+    unsigned long long* c = reinterpret_cast<unsigned long long*>(insts[i].ctl);
+    for (int k = t % 32; k < W; k += 32) {
+        if (SCATTER) c[k] = a[k];
+        else a[k] = c[k];
+    }
+}
+
 // Built solver combinations: 1D hydro {HLLC, exact} x 2D MHD {HLLD} x tile
 // {126, 254} cells (the tile's half states, TS + 2 cells, fill 128 or 256
 // threads of the CTA's round).
@@ -82,6 +101,8 @@ struct dragon_batch {
     size_t ctr_words = 0;
     Summary* d_sum = nullptr;
     Summary* h_sum = nullptr;
+    StepCtl* d_all = nullptr;  // every member's control block (k_batch_ctl)
+    StepCtl* h_all = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     bool dirty = true;
@@ -100,12 +121,16 @@ void release_device(dragon_batch* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     b->gexec = nullptr;
     b->graph = nullptr;
-    for (void* p : {(void*)b->d_insts, (void*)b->d_items, (void*)b->d_ctr, (void*)b->d_sum, (void*)b->d_fmembers})
+    for (void* p : {(void*)b->d_insts, (void*)b->d_items, (void*)b->d_ctr, (void*)b->d_sum, (void*)b->d_fmembers,
+                    (void*)b->d_all})
         if (p) cudaFree(p);
     b->d_fmembers = nullptr;
     b->n_fmembers = 0;
     b->fuse_ctas = 0;
     if (b->h_sum) cudaFreeHost(b->h_sum);
+    if (b->h_all) cudaFreeHost(b->h_all);
+    b->d_all = nullptr;
+    b->h_all = nullptr;
     b->d_insts = nullptr;
     b->d_items = nullptr;
     b->d_ctr = nullptr;
@@ -236,7 +261,23 @@ int build(dragon_batch* b) {
     std::vector<BatchInst> insts;
     insts.reserve(n);
     const bool mixed = b->prec == 1;
-    for (dragon_grid* h : b->members) insts.push_back(make_inst(h, b->tune.tile_1d, b->tune.mhd_tiles, mixed));
+    const StepKernel kern = mixed ? pick_kernel_mx(b->s1d, b->tune.tile_1d) : pick_kernel(b->s1d, b->tune.tile_1d);
+    int dev = 0, sms = 0, occ = 0;
+    CKB(cudaGetDevice(&dev));
+    CKB(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CKB(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, 0));
+    if (occ < 1) return fail(DRAGON_GPU_ECUDA, "batched step kernel cannot be resident");
+    const int per_sm = b->tune.ctas_per_sm > 0 ? std::min(b->tune.ctas_per_sm, occ) : occ;
+    // Tiles of a 2D MHD phase per work item: the tuning's number, fewer where
+    // the members together have too few tiles of a phase for the resident CTAs
+    // (a phase of 8 grids of 80^2 to 160^2 took 100 items of eight tiles, one
+    // after another, on 296 CTAs: 0.57 ms a step against 0.24 with two; 8
+    // grids of 27^2 to 54^2: 0.36 against 0.11 with one)
+    long long tiles = 0;
+    for (dragon_grid* h : b->members)
+        if (h->dim == 2) tiles += (long long)tiles_along(h->n[0] + 4, kTileI) * tiles_along(h->n[1] + 4, kTileJ);
+    const int group = (int)std::max<long long>(1, std::min<long long>(b->tune.mhd_tiles, tiles / (per_sm * sms)));
+    for (dragon_grid* h : b->members) insts.push_back(make_inst(h, b->tune.tile_1d, group, mixed));
     std::vector<int> fmembers;  // a mixed batch's 2D MHD members, in the fused launch's CTA order
     if (mixed) {
         int first = 0;
@@ -257,6 +298,8 @@ int build(dragon_batch* b) {
     CKB(cudaMalloc(&b->d_ctr, sizeof(unsigned) * b->ctr_words));
     CKB(cudaMalloc(&b->d_sum, sizeof(Summary) * n));
     CKB(cudaMallocHost(&b->h_sum, sizeof(Summary) * n));
+    CKB(cudaMalloc(&b->d_all, sizeof(StepCtl) * n));
+    CKB(cudaMallocHost(&b->h_all, sizeof(StepCtl) * n));
     CKB(cudaMemcpyAsync(b->d_insts, insts.data(), sizeof(BatchInst) * n, cudaMemcpyHostToDevice, b->stream));
     if (!q.empty())
         CKB(cudaMemcpyAsync(b->d_items, q.data(), sizeof(WorkItem) * q.size(), cudaMemcpyHostToDevice, b->stream));
@@ -268,13 +311,6 @@ int build(dragon_batch* b) {
     CKB(cudaMemsetAsync(b->d_ctr, 0, sizeof(unsigned) * b->ctr_words, b->stream));
     CKB(cudaStreamSynchronize(b->stream));
 
-    const StepKernel kern = mixed ? pick_kernel_mx(b->s1d, b->tune.tile_1d) : pick_kernel(b->s1d, b->tune.tile_1d);
-    int dev = 0, sms = 0, occ = 0;
-    CKB(cudaGetDevice(&dev));
-    CKB(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CKB(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, 0));
-    if (occ < 1) return fail(DRAGON_GPU_ECUDA, "batched step kernel cannot be resident");
-    int per_sm = b->tune.ctas_per_sm > 0 ? std::min(b->tune.ctas_per_sm, occ) : occ;
     b->grid_ctas = std::max(1, std::min(per_sm * sms, b->nitems));
 
     CKB(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -335,18 +371,21 @@ int advance(dragon_batch* b, int nsteps, dragon_batch_stats* st) {
     if (n == 0 || nsteps == 0) return 0;
     int rc;
     // members' pending work, then each member's control block for this advance
-    for (dragon_grid* h : b->members) CKB(cudaStreamSynchronize(h->stream));
-    for (dragon_grid* h : b->members) {
+    if (b->dirty && (rc = build(b))) return rc;
+    for (int i = 0; i < n; i++) {
+        dragon_grid* h = b->members[i];
         if (!h->imax_valid) {
             if ((rc = zero_slot(h, h->cur))) return rc;
             if ((rc = launch_interior_cfl(h, h->cur, h->cur))) return rc;
         }
         reset_ctl(h, INFINITY, nsteps, 1);
         h->hctl->cur = h->cur;
-        if ((rc = push_ctl(h))) return rc;
+        b->h_all[i] = *h->hctl;
     }
     for (dragon_grid* h : b->members) CKB(cudaStreamSynchronize(h->stream));
-    if (b->dirty && (rc = build(b))) return rc;
+    CKB(cudaMemcpyAsync(b->d_all, b->h_all, sizeof(StepCtl) * n, cudaMemcpyHostToDevice, b->stream));
+    k_batch_ctl<true><<<(n * 32 + 255) / 256, 256, 0, b->stream>>>(b->d_insts, n, b->d_all);
+    CKB(cudaGetLastError());
     CKB(cudaMemsetAsync(b->d_ctr + kCtrTimeouts, 0, sizeof(unsigned), b->stream));
     {
         const unsigned active = (unsigned)n;
@@ -380,9 +419,14 @@ int advance(dragon_batch* b, int nsteps, dragon_batch_stats* st) {
         if (--budget <= 0) return fail(DRAGON_GPU_ESTEP, "batched advance did not finish its steps");
     }
     unsigned timeouts = 0;
-    CKB(cudaMemcpy(&timeouts, b->d_ctr + kCtrTimeouts, sizeof(unsigned), cudaMemcpyDeviceToHost));
-    for (dragon_grid* h : b->members) {
-        if ((rc = pull_ctl(h))) return rc;
+    k_batch_ctl<false><<<(n * 32 + 255) / 256, 256, 0, b->stream>>>(b->d_insts, n, b->d_all);
+    CKB(cudaGetLastError());
+    CKB(cudaMemcpyAsync(b->h_all, b->d_all, sizeof(StepCtl) * n, cudaMemcpyDeviceToHost, b->stream));
+    CKB(cudaMemcpyAsync(&timeouts, b->d_ctr + kCtrTimeouts, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
+    CKB(cudaStreamSynchronize(b->stream));
+    for (int i = 0; i < n; i++) {
+        dragon_grid* h = b->members[i];
+        *h->hctl = b->h_all[i];
         add_newton(h, *h->hctl);
         h->cur = h->hctl->cur;
         h->imax_valid = true;
