@@ -39,6 +39,7 @@ struct AdvanceState {
     int retries = 0;
     double remaining = 0;
     int max_steps = 0;
+    bool check_cfl = true;
 };
 
 struct dragon_grid {
@@ -93,6 +94,10 @@ struct dragon_grid {
     dgpu::MlpNet* mlp_dev = nullptr;
     dragon_newton_stats ntot{};
     AdvanceState adv{};
+    // the CFL dt last read back (0: none): how many steps an interval is likely
+    // to take, so that a batch enqueues no more. A guess only: it decides how
+    // many steps are enqueued at a time, never their dt.
+    double dt_hint = 0;
     // CTAs of the cooperative prologue that fit on the device (hydro, MHD); 0: not yet known, -1: none
     int coop_cap[2] = {0, 0};
     // test hooks (dragon_gpu_debug_set): CTA of the cooperative prologue that

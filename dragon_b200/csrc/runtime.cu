@@ -318,9 +318,12 @@ static int launch_prologue_range(dragon_grid* h, int c, int bookkeeping, int app
     pa.nbc = bc_count;
     pa.bc_first = bc_first;
     pa.stall_cta = h->dbg_stall_cta;
+    // a 1D grid has a few ghost cells and two ring cells: one warp, whose block
+    // reductions and barriers cost next to nothing
+    const int nt = h->dim == 1 ? 32 : 1024;
     auto one_cta = [&](const PrologueArgs& a) {
-        if (h->mhd) k_prologue<true><<<1, 1024, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
-        else k_prologue<false><<<1, 1024, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
+        if (h->mhd) k_prologue<true><<<1, nt, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
+        else k_prologue<false><<<1, nt, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
         h->launches++;
     };
     // 2D / 3D: one pass over the ghost shell where the list allows it; with no
@@ -569,9 +572,17 @@ const char* stage_name(int s) {
 // One batch of up to kBatch steps of the advance in flight: for step k the
 // prologue (bookkeeping, ghost fill, CFL dt) reads buffer cur0 ^ (k & 1) and
 // the step writes the other buffer.
-static int enqueue_batch(dragon_grid* h) {
+//
+// An interval's batches hold the steps it should still take at the last known
+// CFL dt `left` / dt_hint (a step more that the dt turns out to need costs
+// another batch, one too many two empty launches): a full batch of 64 for the
+// one step of advance(cfl_time()) cost 0.4 ms of launches on a 96^2 grid whose
+// step takes 0.03.
+static int enqueue_batch(dragon_grid* h, double left) {
     AdvanceState& A = h->adv;
     int nb = kBatch;
+    if (A.max_steps <= 0 && !A.check_cfl) nb = 1;  // the interval is one step
+    else if (A.max_steps <= 0) nb = h->dt_hint > 0 ? (int)std::min<double>(kBatch, std::ceil(left / h->dt_hint)) : 4;
     if (A.max_steps > 0) nb = (int)std::min<long long>(kBatch, (long long)A.max_steps + 1 - A.k);
     if (nb < 1) nb = 1;
     int rc;
@@ -602,6 +613,12 @@ static bool account_last_step(dragon_grid* h, StepCtl& C) {
     return C.done != 0;
 }
 
+// Keeps the CFL dt of a control block that was read back.
+static void note_dt(dragon_grid* h, const StepCtl& C) {
+    const double dt = h->cfg.cfl_coeff * (h->dim == 1 ? h->d[0] : 1.0) / C.max_speed;
+    if (C.max_speed > 0 && std::isfinite(dt)) h->dt_hint = dt;
+}
+
 int advance_begin(dragon_grid* h, double remaining, int max_steps, int check_cfl) {
     if (h->adv.pending) return fail(DRAGON_GPU_EINVAL, "an asynchronous advance is in flight: call dragon_gpu_advance_wait");
     h->can_rollback = false;
@@ -610,6 +627,7 @@ int advance_begin(dragon_grid* h, double remaining, int max_steps, int check_cfl
     A.cur0 = h->cur;
     A.remaining = remaining;
     A.max_steps = max_steps;
+    A.check_cfl = check_cfl != 0;
     reset_ctl(h, remaining, max_steps, check_cfl);
     int rc = push_ctl(h);
     if (rc) return rc;
@@ -618,7 +636,7 @@ int advance_begin(dragon_grid* h, double remaining, int max_steps, int check_cfl
         if ((rc = launch_interior_cfl(h, A.cur0, A.cur0))) return rc;
     }
     A.pending = true;
-    rc = enqueue_batch(h);
+    rc = enqueue_batch(h, remaining);
     if (rc) A.pending = false;
     return rc;
 }
@@ -636,6 +654,7 @@ int advance_finish(dragon_grid* h, dragon_advance_stats* st) {
     for (;;) {
         if ((rc = pull_ctl(h))) return rc;
         StepCtl& C = *h->hctl;
+        note_dt(h, C);
         if (C.err) {
             const long long ks = C.steps_done;  // index of the failed step
             const int c = cur0 ^ (int)(ks & 1);
@@ -680,11 +699,15 @@ int advance_finish(dragon_grid* h, dragon_advance_stats* st) {
             // success: the next prologue accounts the retried step; step k reads
             // buffer cur0 ^ (k & 1) == c ^ 1
             A.k = ks + 1;
-            if ((rc = enqueue_batch(h))) return rc;
+            if ((rc = enqueue_batch(h, C.remaining - C.t1))) return rc;
             continue;
         }
         if (!C.done && A.max_steps > 0 && A.k > A.max_steps && !account_last_step(h, C))
             return fail(DRAGON_GPU_ESTEP, "step budget consumed but the advance did not finish");
+        // an interval that the batch's last step used up ends here, without the
+        // prologue that would find it so
+        if (!C.done && A.max_steps <= 0 && C.have_prev && !(C.remaining - C.t1 > h->cfg.timestep_tol))
+            account_last_step(h, C);
         if (C.done) {
             h->cur = cur0 ^ (int)(C.steps_done & 1);
             h->imax_valid = true;
@@ -700,7 +723,7 @@ int advance_finish(dragon_grid* h, dragon_advance_stats* st) {
             }
             return 0;
         }
-        if ((rc = enqueue_batch(h))) return rc;
+        if ((rc = enqueue_batch(h, C.remaining - C.t1))) return rc;
     }
 }
 
@@ -1009,6 +1032,7 @@ int dragon_gpu_cfl_time(dragon_grid* h, double* dt_out) {
     if ((rc = launch_prologue(h, h->cur, 0, 0, 1, 2, 2))) return rc;
     if ((rc = pull_ctl(h))) return rc;
     if (h->hctl->err) return fail(DRAGON_GPU_ECFL, stage_name(ST_CFL_ZERO));
+    note_dt(h, *h->hctl);
     *dt_out = h->hctl->t1;
     return 0;
 }
