@@ -14,24 +14,50 @@ namespace dgpu {
 // one instruction sequence with a runtime direction 0.294.
 constexpr int k2dTI = 14, k2dTJ = 26, k2dNT = 256;
 
-template <int S>
-static int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, const CUtensorMap* map,
-              cudaStream_t st) {
-    auto kern = k_step2d_hydro<S, k2dTI, k2dTJ, k2dNT>;
-    const size_t smem = sizeof(Smem2DH<k2dTI, k2dTJ>);
+// A grid whose large tiles do not fill the GPU waits for the longest CTA, not
+// for its arithmetic, so smaller grids take smaller tiles: 6 x 30 cells, whose
+// 256 half states are one round of the threads (faces and corrections two),
+// and 6 x 14, whose every phase is one round (128 half states, 232 and 188
+// faces, 208 corrections, 84 updates). Step times in us, 6 x 14 / 6 x 30 / 14 x
+// 26 cells: 96^2 22.6 / 24.7 / 32.9, 128^2 25.6 / 25.7 / 33.9, 200^2 35.6 / 31.0
+// / 33.1, 320^2 61.6 / 51.1 / 56.2, 400^2 85 / 68.5 / 68.6, 512^2 128 / 96 / 82.
+// Hence the lines: 6 x 14 up to one CTA per SM, 6 x 30 up to five.
+enum Tile2D { kTile14x26, kTile6x30, kTile6x14 };
+static Tile2D pick_tile(const Geo& G) {
+    auto ctas = [&](int ti, int tj) { return (long long)((G.n[0] + ti - 1) / ti) * ((G.n[1] + tj - 1) / tj); };
+    if (ctas(6, 14) <= 148) return kTile6x14;
+    if (ctas(6, 30) <= 148 * 5) return kTile6x30;
+    return kTile14x26;
+}
+
+template <int S, int TI, int TJ>
+static int go_tile(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa,
+                   const CUtensorMap* map, cudaStream_t st) {
+    auto kern = k_step2d_hydro<S, TI, TJ, k2dNT>;
+    const size_t smem = sizeof(Smem2DH<TI, TJ>);
     static bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 1;
         attr_set = true;
     }
-    dim3 grid((G.n[1] + k2dTJ - 1) / k2dTJ, (G.n[0] + k2dTI - 1) / k2dTI);
+    dim3 grid((G.n[1] + TJ - 1) / TJ, (G.n[0] + TI - 1) / TI);
     kern<<<grid, k2dNT, smem, st>>>(G, win, wout, ctl, sa, *map);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
+template <int S>
+static int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, const CUtensorMap* map,
+              cudaStream_t st) {
+    switch (pick_tile(G)) {
+        case kTile6x14: return go_tile<S, 6, 14>(G, win, wout, ctl, sa, map, st);
+        case kTile6x30: return go_tile<S, 6, 30>(G, win, wout, ctl, sa, map, st);
+        default: return go_tile<S, k2dTI, k2dTJ>(G, win, wout, ctl, sa, map, st);
+    }
+}
 
-int step2d_tile_box(int mixed, int box[3]) {
-    box[0] = (mixed ? kMx2dTJ : k2dTJ) + 6;
-    box[1] = (mixed ? kMx2dTI : k2dTI) + 4;
+int step2d_tile_box(int mixed, const Geo& G, int box[3]) {
+    const Tile2D t = pick_tile(G);
+    box[0] = (mixed ? kMx2dTJ : t == kTile6x14 ? 14 : t == kTile6x30 ? 30 : k2dTJ) + 6;
+    box[1] = (mixed ? kMx2dTI : t == kTile14x26 ? k2dTI : 6) + 4;
     box[2] = 5;
     return 0;
 }

@@ -228,7 +228,7 @@ static int state_tile_map(dragon_grid* h, int mixed, int b, const CUtensorMap** 
         auto encode = tensor_map_encoder();
         if (!encode) return fail(DRAGON_GPU_ECUDA, "cuTensorMapEncodeTiled is not available");
         int box[3];
-        step2d_tile_box(mixed, box);
+        step2d_tile_box(mixed, h->cg, box);
         const cuuint64_t dims[3] = {(cuuint64_t)h->cg.ext[1], (cuuint64_t)h->cg.ext[0], 5};
         const cuuint64_t strides[2] = {(cuuint64_t)h->cg.pitch * sizeof(double), (cuuint64_t)h->cg.plane * sizeof(double)};
         const cuuint32_t boxd[3] = {(cuuint32_t)box[0], (cuuint32_t)box[1], (cuuint32_t)box[2]};
