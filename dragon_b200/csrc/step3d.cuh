@@ -70,7 +70,9 @@ __device__ __forceinline__ void stc5(double* a, long long P, long long m, const 
 }
 
 // K1: MUSCL half states along all three axes (computeHalfStates_X/Y/Z, Unsplit.cpp:344-436).
-static __global__ void k_h3_halfstates(Step3DArgs A) {
+// Three CTAs per SM, here and in the update (98 and 96 registers unbounded,
+// two CTAs: 1 % slower steps): both wait on memory more than on FP64.
+static __global__ void __launch_bounds__(256, 3) k_h3_halfstates(Step3DArgs A) {
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -432,7 +434,7 @@ __global__ void __launch_bounds__(256, 2) k_h3_final(Step3DArgs A) {
 
 // K5: conservative update of the interior (applyFluxes 3D, Unsplit.cpp:272-288),
 // physicality, CFL speed of the committed state.
-static __global__ void k_h3_update(Step3DArgs A) {
+static __global__ void __launch_bounds__(256, 3) k_h3_update(Step3DArgs A) {
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;

@@ -186,8 +186,10 @@ __device__ __forceinline__ V3 m3_edge_e(const Mhd3DArgs& A, const double* __rest
 
 // K3 (edges [-1, n+1]^3, against the body E of w) and K6 (edges [0, n]^3,
 // against the half-step body E).
+// Loads alone: four CTAs per SM (and two for k_m3_update, 130 registers
+// unbounded; both together 1.5 % of the 96^3 step).
 template <bool FINAL>
-__global__ void k_m3_edges(Mhd3DArgs A) {
+__global__ void __launch_bounds__(256, 4) k_m3_edges(Mhd3DArgs A) {
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -298,7 +300,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
 }
 
 // K7
-static __global__ void k_m3_update(Mhd3DArgs A) {
+static __global__ void __launch_bounds__(256, 2) k_m3_update(Mhd3DArgs A) {
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;
