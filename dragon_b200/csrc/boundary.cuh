@@ -10,6 +10,7 @@
 // Periodic.cpp:311-331, Fixed.cpp:372-406).
 #pragma once
 
+#include "chain.cuh"
 #include "grid.cuh"
 
 namespace dgpu {
@@ -377,6 +378,7 @@ __device__ __forceinline__ void prologue_body(const Geo& G, const Geo& FG, doubl
 template <bool MHD>
 __global__ void __launch_bounds__(1024) k_prologue(Geo G, Geo FG, double* __restrict__ w, double* __restrict__ B,
                                                    const BCEntry* __restrict__ bcs, StepCtl* ctl, PrologueArgs pa) {
+    chained();
     prologue_body<MHD>(G, FG, w, B, bcs, ctl, pa);
 }
 
@@ -528,52 +530,6 @@ inline bool direct_fill_ok(const Geo& G, const BCEntry* e, int first, int count,
     return true;
 }
 
-// Item t of the points of a padded box outside its interior [0, n): lo layers
-// below and hi above along every axis. False past the last.
-struct ShellBox {
-    int n[3], lo, hi, dim;
-    unsigned s0, s1, total;  // items of the first axis' slabs, of the first two
-};
-__host__ __device__ __forceinline__ ShellBox shell_box(const Geo& G, const int* n, int lo, int hi) {
-    ShellBox b;
-    b.dim = G.dim;
-    b.lo = lo;
-    b.hi = hi;
-    for (int a = 0; a < 3; a++) b.n[a] = a < G.dim ? n[a] : 1;
-    const unsigned w = lo + hi;
-    const unsigned e1 = G.dim > 1 ? n[1] + w : 1, e2 = G.dim > 2 ? n[2] + w : 1;
-    b.s0 = w * e1 * e2;
-    b.s1 = b.s0 + (unsigned)b.n[0] * w * e2;
-    b.total = G.dim > 2 ? b.s1 + (unsigned)b.n[0] * b.n[1] * w : b.s1;
-    return b;
-}
-__device__ __forceinline__ void shell_point(const ShellBox& b, unsigned t, int* c) {
-    const unsigned w = b.lo + b.hi;
-    const unsigned e1 = b.n[1] + w, e2 = b.dim > 2 ? b.n[2] + w : 1;
-    auto layer = [&](unsigned l, int n) { return (int)l < b.lo ? (int)l - b.lo : n + (int)l - b.lo; };
-    if (t < b.s0) {
-        const unsigned q = t / e2, k = t - q * e2;
-        c[0] = layer(q / e1, b.n[0]);
-        c[1] = (int)(q % e1) - b.lo;
-        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
-    } else if (t < b.s1) {
-        t -= b.s0;
-        const unsigned q = t / e2, k = t - q * e2;
-        c[0] = q / w;
-        c[1] = layer(q % w, b.n[1]);
-        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
-    } else {
-        t -= b.s1;
-        const unsigned q = t / w;
-        c[2] = layer(t - q * w, b.n[2]);
-        c[0] = q / b.n[1];
-        c[1] = q % b.n[1];
-    }
-}
-__device__ __forceinline__ long long gidx(const Geo& G, const int* c) {
-    return G.dim == 2 ? gidx2(G, c[0], c[1]) : gidx3(G, c[0], c[1], c[2]);
-}
-
 // The value of ghost cell c after every pass of the list; false if none writes it.
 template <bool MHD>
 __device__ __forceinline__ bool direct_cell(const Geo& G, const double* __restrict__ w, const DirectList& list,
@@ -693,6 +649,7 @@ template <bool MHD>
 __global__ void __launch_bounds__(128) k_prologue_direct(Geo G, Geo FG, double* __restrict__ w, double* __restrict__ B,
                                                          const __grid_constant__ DirectList list, StepCtl* ctl,
                                                          PrologueArgs pa, ShellBox cells, ShellBox faces) {
+    chained();
     __shared__ int s_skip;
     __shared__ double s_red[32];
     if (threadIdx.x == 0) s_skip = *(const volatile int*)&ctl->err ? 1 : bookkeeping_done(ctl, pa) ? 2 : 0;

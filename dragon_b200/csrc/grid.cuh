@@ -37,6 +37,67 @@ __device__ __forceinline__ long long gidx3(const Geo& G, int i, int j, int k) {
     return (long long)(i + G.g) * G.pitch2 + (long long)(j + G.g) * G.pitch + (k + G.g);
 }
 
+// Item t of the points of a padded box outside its interior [0, n): lo layers
+// below and hi above along every axis. False past the last.
+struct ShellBox {
+    int n[3], lo, hi, dim;
+    unsigned s0, s1, total;  // items of the first axis' slabs, of the first two
+};
+__host__ __device__ __forceinline__ ShellBox shell_box(const Geo& G, const int* n, int lo, int hi) {
+    ShellBox b;
+    b.dim = G.dim;
+    b.lo = lo;
+    b.hi = hi;
+    for (int a = 0; a < 3; a++) b.n[a] = a < G.dim ? n[a] : 1;
+    const unsigned w = lo + hi;
+    const unsigned e1 = G.dim > 1 ? n[1] + w : 1, e2 = G.dim > 2 ? n[2] + w : 1;
+    b.s0 = w * e1 * e2;
+    b.s1 = b.s0 + (unsigned)b.n[0] * w * e2;
+    b.total = G.dim > 2 ? b.s1 + (unsigned)b.n[0] * b.n[1] * w : b.s1;
+    return b;
+}
+__device__ __forceinline__ void shell_point(const ShellBox& b, unsigned t, int* c) {
+    const unsigned w = b.lo + b.hi;
+    const unsigned e1 = b.n[1] + w, e2 = b.dim > 2 ? b.n[2] + w : 1;
+    auto layer = [&](unsigned l, int n) { return (int)l < b.lo ? (int)l - b.lo : n + (int)l - b.lo; };
+    if (t < b.s0) {
+        const unsigned q = t / e2, k = t - q * e2;
+        c[0] = layer(q / e1, b.n[0]);
+        c[1] = (int)(q % e1) - b.lo;
+        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
+    } else if (t < b.s1) {
+        t -= b.s0;
+        const unsigned q = t / e2, k = t - q * e2;
+        c[0] = q / w;
+        c[1] = layer(q % w, b.n[1]);
+        c[2] = b.dim > 2 ? (int)k - b.lo : 0;
+    } else {
+        t -= b.s1;
+        const unsigned q = t / w;
+        c[2] = layer(t - q * w, b.n[2]);
+        c[0] = q / b.n[1];
+        c[1] = q % b.n[1];
+    }
+}
+__device__ __forceinline__ long long gidx(const Geo& G, const int* c) {
+    return G.dim == 2 ? gidx2(G, c[0], c[1]) : gidx3(G, c[0], c[1], c[2]);
+}
+
+// Copies NF planes at every point of a padded box outside its interior, by
+// thread tid of nthr: the ghost part of a step's output, which the committed
+// arrays keep (Unsplit.cpp:106 commits the interior only).
+template <int NF>
+__device__ __forceinline__ void copy_shell(const Geo& G, const ShellBox& b, const double* __restrict__ in,
+                                           double* __restrict__ out, unsigned tid, unsigned nthr) {
+    for (unsigned t = tid; t < b.total; t += nthr) {
+        int c[3];
+        shell_point(b, t, c);
+        const long long m = gidx(G, c);
+#pragma unroll
+        for (int f = 0; f < NF; f++) out[f * G.plane + m] = in[f * G.plane + m];
+    }
+}
+
 // Mutable per-grid state the kernels of one advance share. Lives in device
 // memory; the host reads it back after a batch of steps.
 struct StepCtl {

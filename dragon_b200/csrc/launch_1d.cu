@@ -1,4 +1,5 @@
 // 1D sweep launchers (hydro and MHD, every solver).
+#include "chain.cuh"
 #include "launchers.h"
 #include "step_hydro.cuh"
 
@@ -18,7 +19,7 @@ template <bool MHD, int S>
 static int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, cudaStream_t st) {
     const int np = G.n[0] + 2 * G.g;
     constexpr int TS = Tile1D<MHD>::TS, NT = Tile1D<MHD>::NT;
-    k_step1d<MHD, S, TS, NT><<<(np + TS - 1) / TS, NT, 0, st>>>(G, win, wout, ctl, sa);
+    chain(k_step1d<MHD, S, TS, NT>, (np + TS - 1) / TS, NT, 0, st, G, win, wout, ctl, sa);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

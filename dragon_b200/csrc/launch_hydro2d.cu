@@ -1,4 +1,5 @@
 // FP64 fused 2D CTU hydro launchers (every hydro solver).
+#include "chain.cuh"
 #include "launchers.h"
 #include "step_hydro.cuh"
 
@@ -41,7 +42,7 @@ static int go_tile(const Geo& G, const double* win, double* wout, StepCtl* ctl, 
         attr_set = true;
     }
     dim3 grid((G.n[1] + TJ - 1) / TJ, (G.n[0] + TI - 1) / TI);
-    kern<<<grid, k2dNT, smem, st>>>(G, win, wout, ctl, sa, *map);
+    chain(kern, grid, k2dNT, smem, st, G, win, wout, ctl, sa, *map);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 template <int S>

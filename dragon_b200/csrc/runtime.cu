@@ -22,6 +22,7 @@
 
 #include "../../include/dragon_gpu.h"
 #include "../../include/dragon_learned.h"
+#include "chain.cuh"
 #include "boundary.cuh"
 #include "handle.h"
 #include "launchers.h"
@@ -322,8 +323,8 @@ static int launch_prologue_range(dragon_grid* h, int c, int bookkeeping, int app
     // reductions and barriers cost next to nothing
     const int nt = h->dim == 1 ? 32 : 1024;
     auto one_cta = [&](const PrologueArgs& a) {
-        if (h->mhd) k_prologue<true><<<1, nt, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
-        else k_prologue<false><<<1, nt, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
+        if (h->mhd) chain(k_prologue<true>, 1, nt, 0, h->stream, h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
+        else chain(k_prologue<false>, 1, nt, 0, h->stream, h->cg, h->fg, W, h->B[c], h->dbcs, h->ctl, a);
         h->launches++;
     };
     // 2D / 3D: one pass over the ghost shell where the list allows it; with no
@@ -337,9 +338,9 @@ static int launch_prologue_range(dragon_grid* h, int c, int bookkeeping, int app
         const unsigned items = cells.total + (h->mhd && apply_bc ? faces.total : 0);
         const int blocks = (int)std::min<unsigned>((items + 127) / 128, 148 * 16);
         if (h->mhd)
-            k_prologue_direct<true><<<blocks, 128, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
+            chain(k_prologue_direct<true>, blocks, 128, 0, h->stream, h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
         else
-            k_prologue_direct<false><<<blocks, 128, 0, h->stream>>>(h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
+            chain(k_prologue_direct<false>, blocks, 128, 0, h->stream, h->cg, h->fg, W, h->B[c], list, h->ctl, pa, cells, faces);
         CK(cudaGetLastError());
         h->launches++;
         return 0;

@@ -1,6 +1,7 @@
 // Single-grid mixed FP32/FP64 1D sweeps: step1d_tile_mx (hydro) and
 // step1d_tile_mx_mhd (MHD) of step1d_mixed.cuh, one tile per CTA. Compiled with FMA contraction and
 // fast single-precision division / square root.
+#include "chain.cuh"
 #include "launchers.h"
 #include "step1d_mixed.cuh"
 
@@ -11,6 +12,7 @@ namespace {
 template <int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT)
 k_step1d_mx(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+    chained();
     step1d_tile_mx<SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }
 
@@ -19,6 +21,7 @@ k_step1d_mx(Geo G, const double* __restrict__ win, double* __restrict__ wout, St
 template <int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT)
 k_step1d_mx_mhd(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+    chained();
     step1d_tile_mx_mhd<SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }
 
@@ -26,15 +29,14 @@ template <int S>
 int go_mhd(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, cudaStream_t st) {
     constexpr int TS = 126, NT = 128;
     const int np = G.n[0] + 2 * G.g;
-    k_step1d_mx_mhd<S, TS, NT><<<(np + TS - 1) / TS, NT, 0, st>>>(G, win, wout, ctl, sa);
+    chain(k_step1d_mx_mhd<S, TS, NT>, (np + TS - 1) / TS, NT, 0, st, G, win, wout, ctl, sa);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
 template <int S>
 int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const StepArgs& sa, cudaStream_t st) {
     const int np = G.n[0] + 2 * G.g;
-    k_step1d_mx<S, kMx1dTile, kMx1dThreads><<<(np + kMx1dTile - 1) / kMx1dTile, kMx1dThreads, 0, st>>>(G, win, wout,
-                                                                                                    ctl, sa);
+    chain(k_step1d_mx<S, kMx1dTile, kMx1dThreads>, (np + kMx1dTile - 1) / kMx1dTile, kMx1dThreads, 0, st, G, win, wout, ctl, sa);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

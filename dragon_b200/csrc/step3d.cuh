@@ -12,6 +12,7 @@
 // Index ranges are the reference's, so every Riemann pivot that can fail does.
 #pragma once
 
+#include "chain.cuh"
 #include "grid.cuh"
 #include "mlp.cuh"
 #include "recon.cuh"
@@ -73,8 +74,11 @@ __device__ __forceinline__ void stc5(double* a, long long P, long long m, const 
 // Three CTAs per SM, here and in the update (98 and 96 registers unbounded,
 // two CTAs: 1 % slower steps): both wait on memory more than on FP64.
 static __global__ void __launch_bounds__(256, 3) k_h3_halfstates(Step3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
+    copy_shell<5>(A.G, shell_box(A.G, A.G.n, A.G.g, A.G.g), A.w, A.wout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
     const Geo& G = A.G;
     const int lo[3] = {-1, -1, -1}, ext[3] = {G.n[0] + 2, G.n[1] + 2, G.n[2] + 2};
     int i, j, k;
@@ -336,6 +340,7 @@ static __global__ void k_h3_final_learned(Step3DArgs A) {
 // registers unbounded (one CTA per SM) and ran 33 % faster capped at 128.
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 2) k_h3_prelim(Step3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -380,6 +385,7 @@ __device__ __forceinline__ void h3_ctu_flux(const Step3DArgs& A, const double* T
 // third axis cells [-1, n].
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 2) k_h3_ctu(Step3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -416,6 +422,7 @@ __global__ void __launch_bounds__(256, 2) k_h3_ctu(Step3DArgs A) {
 // range (x states: cells [-1,nx] x [0,ny) x [0,nz), and likewise).
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 2) k_h3_final(Step3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -435,6 +442,7 @@ __global__ void __launch_bounds__(256, 2) k_h3_final(Step3DArgs A) {
 // K5: conservative update of the interior (applyFluxes 3D, Unsplit.cpp:272-288),
 // physicality, CFL speed of the committed state.
 static __global__ void __launch_bounds__(256, 3) k_h3_update(Step3DArgs A) {
+    chained();
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;
@@ -471,21 +479,20 @@ inline int launch_step3d_hydro_t(const Geo& G, const double* w, double* wout, co
     const long long box = (long long)(G.n[0] + 2) * (G.n[1] + 2) * (G.n[2] + 2);
     const long long fbox = (long long)(G.n[0] + 1) * (G.n[1] + 1) * (G.n[2] + 1);
     const long long cells = (long long)G.n[0] * G.n[1] * G.n[2];
-    if (cudaMemcpyAsync(wout, w, sizeof(double) * 5 * G.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    k_h3_halfstates<<<blocks(box), 256, 0, st>>>(A);
+    chain(k_h3_halfstates, blocks(box), 256, 0, st, A);
     if constexpr (SOLVER == RS_EXACT) {
         if (learned) {
             k_h3_prelim_learned<<<blocks(box), 256, 0, st>>>(A);
             k_h3_ctu_learned<<<blocks(box), 256, 0, st>>>(A);
             k_h3_final_learned<<<blocks(fbox), 256, 0, st>>>(A);
-            k_h3_update<<<blocks(cells), 256, 0, st>>>(A);
+            chain(k_h3_update, blocks(cells), 256, 0, st, A);
             return cudaGetLastError() == cudaSuccess ? 0 : 1;
         }
     }
-    k_h3_prelim<SOLVER><<<blocks(box), 256, 0, st>>>(A);
-    k_h3_ctu<SOLVER><<<blocks(box), 256, 0, st>>>(A);
-    k_h3_final<SOLVER><<<blocks(fbox), 256, 0, st>>>(A);
-    k_h3_update<<<blocks(cells), 256, 0, st>>>(A);
+    chain(k_h3_prelim<SOLVER>, blocks(box), 256, 0, st, A);
+    chain(k_h3_ctu<SOLVER>, blocks(box), 256, 0, st, A);
+    chain(k_h3_final<SOLVER>, blocks(fbox), 256, 0, st, A);
+    chain(k_h3_update, blocks(cells), 256, 0, st, A);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

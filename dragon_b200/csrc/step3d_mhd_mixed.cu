@@ -12,6 +12,7 @@
 // operand roles and failure points are those of the FP64 step. Compiled with
 // FMA contraction and fast single-precision division / square root, like the
 // other mixed translation units.
+#include "chain.cuh"
 #include "launchers.h"
 #include "mixed.cuh"
 #include "step_mhd3d.cuh"
@@ -64,8 +65,13 @@ __device__ __forceinline__ Prim<float> f32_prim8(const Prim<double>& w) {
 // Launch bounds: three CTAs per SM spilled the MUSCL and HLLD kernels; two
 // CTAs (128 registers) keep them in registers.
 __global__ void __launch_bounds__(256, 2) k_m3m_halfstates(Mhd3DArgs A, Mx3M X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
+    copy_shell<8>(A.G, shell_box(A.G, A.G.n, A.G.g, A.G.g), A.w, A.wout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
+    copy_shell<3>(A.FG, shell_box(A.FG, A.G.n, A.G.g, A.G.g + 1), A.B, A.Bout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
     int i, j, k;
     if (!m3_cell(blockIdx.x * (long long)blockDim.x + threadIdx.x, -2, 1, A.G, i, j, k)) return;
     const double dt = *(const volatile double*)&A.ctl->t1;
@@ -128,6 +134,7 @@ __device__ __forceinline__ void m3m_face_flux(const Mhd3DArgs& A, const Mx3M& X,
 // K2 (box [-2, n+1]^3) and K5 (box [-1, n]^3).
 template <int SOLVER, bool FINAL>
 __global__ void __launch_bounds__(256, SOLVER == RS_HLLD ? 2 : 3) k_m3m_fluxes(Mhd3DArgs A, Mx3M X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -178,6 +185,7 @@ __device__ __forceinline__ V3 m3m_edge_e(const Mhd3DArgs& A, const Mx3M& X, cons
 // against the half-step body E).
 template <bool FINAL>
 __global__ void k_m3m_edges(Mhd3DArgs A, Mx3M X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -189,6 +197,7 @@ __global__ void k_m3m_edges(Mhd3DArgs A, Mx3M X) {
 // accumulation of the FP32 predictor fluxes) with its body E, and the CTU
 // corrections of the six half states in FP32 with the energies in FP64.
 __global__ void __launch_bounds__(256, 2) k_m3m_half(Mhd3DArgs A, Mx3M X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -278,6 +287,7 @@ __global__ void __launch_bounds__(256, 2) k_m3m_half(Mhd3DArgs A, Mx3M X) {
 // faces the cell owns (FP64), face -> cell B with the energy gate,
 // physicality, CFL speed.
 __global__ void __launch_bounds__(256) k_m3m_update(Mhd3DArgs A, Mx3M X) {
+    chained();
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;
@@ -330,15 +340,13 @@ int go(const Geo& G, const Geo& FG, const double* w, double* wout, const double*
         const long long n = (long long)(G.n[0] + hi - lo + 1) * (G.n[1] + hi - lo + 1) * (G.n[2] + hi - lo + 1);
         return (int)((n + 255) / 256);
     };
-    if (cudaMemcpyAsync(wout, w, sizeof(double) * 8 * G.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    if (cudaMemcpyAsync(Bout, B, sizeof(double) * 3 * FG.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    k_m3m_halfstates<<<blocks(-2, 1), 256, 0, st>>>(A, X);
-    k_m3m_fluxes<SOLVER, false><<<blocks(-2, 1), 256, 0, st>>>(A, X);
-    k_m3m_edges<false><<<blocks(-1, 1), 256, 0, st>>>(A, X);
-    k_m3m_half<<<blocks(-1, 0), 256, 0, st>>>(A, X);
-    k_m3m_fluxes<SOLVER, true><<<blocks(-1, 0), 256, 0, st>>>(A, X);
-    k_m3m_edges<true><<<blocks(0, 0), 256, 0, st>>>(A, X);
-    k_m3m_update<<<blocks(0, -1), 256, 0, st>>>(A, X);
+    chain(k_m3m_halfstates, blocks(-2, 1), 256, 0, st, A, X);
+    chain(k_m3m_fluxes<SOLVER, false>, blocks(-2, 1), 256, 0, st, A, X);
+    chain(k_m3m_edges<false>, blocks(-1, 1), 256, 0, st, A, X);
+    chain(k_m3m_half, blocks(-1, 0), 256, 0, st, A, X);
+    chain(k_m3m_fluxes<SOLVER, true>, blocks(-1, 0), 256, 0, st, A, X);
+    chain(k_m3m_edges<true>, blocks(0, 0), 256, 0, st, A, X);
+    chain(k_m3m_update, blocks(0, -1), 256, 0, st, A, X);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

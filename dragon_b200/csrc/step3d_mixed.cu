@@ -10,6 +10,7 @@
 // order of the corrections and the retry-relevant failure points are those of
 // the FP64 step. Compiled with FMA contraction and fast single-precision
 // division / square root, like the other mixed translation units.
+#include "chain.cuh"
 #include "launchers.h"
 #include "mixed.cuh"
 #include "step3d.cuh"
@@ -46,8 +47,11 @@ __device__ __forceinline__ Prim<float> f32_prim(const Prim<double>& w) {
 
 // K1: MUSCL half states along x, y, z for cells [-1, n]^3.
 __global__ void __launch_bounds__(256, 3) k_h3m_halfstates(Step3DArgs A, Mx3 X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
+    copy_shell<5>(A.G, shell_box(A.G, A.G.n, A.G.g, A.G.g), A.w, A.wout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
     const Geo& G = A.G;
     const int lo[3] = {-1, -1, -1}, ext[3] = {G.n[0] + 2, G.n[1] + 2, G.n[2] + 2};
     int i, j, k;
@@ -97,6 +101,7 @@ __device__ __forceinline__ void h3m_flux(const Step3DArgs& A, const Mx3& X, floa
 // K2: predictor fluxes (CTU.cpp:230-232).
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 3) k_h3m_prelim(Step3DArgs A, Mx3 X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -134,6 +139,7 @@ __device__ __forceinline__ void h3m_ctu_flux(const Step3DArgs& A, const Mx3& X, 
 // K3: the six corner-corrected fluxes over the reference's ranges.
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 3) k_h3m_ctu(Step3DArgs A, Mx3 X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -204,6 +210,7 @@ __device__ __forceinline__ void h3m_final_flux(const Step3DArgs& A, const Mx3& X
 // K4: final fluxes from the corrected half states.
 template <int SOLVER>
 __global__ void __launch_bounds__(256, 3) k_h3m_final(Step3DArgs A, Mx3 X) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     const Geo& G = A.G;
@@ -223,6 +230,7 @@ __global__ void __launch_bounds__(256, 3) k_h3m_final(Step3DArgs A, Mx3 X) {
 // K5: FP64 accumulation of the FP32 flux differences into the FP64 state,
 // FP64 pressure recovery, physicality, CFL speed of the committed state.
 __global__ void __launch_bounds__(256) k_h3m_update(Step3DArgs A, Mx3 X) {
+    chained();
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;
@@ -264,12 +272,11 @@ int go(const Geo& G, const double* w, double* wout, const Hydro3DScratch& S, Ste
     const long long box = (long long)(G.n[0] + 2) * (G.n[1] + 2) * (G.n[2] + 2);
     const long long fbox = (long long)(G.n[0] + 1) * (G.n[1] + 1) * (G.n[2] + 1);
     const long long cells = (long long)G.n[0] * G.n[1] * G.n[2];
-    if (cudaMemcpyAsync(wout, w, sizeof(double) * 5 * G.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    k_h3m_halfstates<<<blocks(box), 256, 0, st>>>(A, X);
-    k_h3m_prelim<SOLVER><<<blocks(box), 256, 0, st>>>(A, X);
-    k_h3m_ctu<SOLVER><<<blocks(box), 256, 0, st>>>(A, X);
-    k_h3m_final<SOLVER><<<blocks(fbox), 256, 0, st>>>(A, X);
-    k_h3m_update<<<blocks(cells), 256, 0, st>>>(A, X);
+    chain(k_h3m_halfstates, blocks(box), 256, 0, st, A, X);
+    chain(k_h3m_prelim<SOLVER>, blocks(box), 256, 0, st, A, X);
+    chain(k_h3m_ctu<SOLVER>, blocks(box), 256, 0, st, A, X);
+    chain(k_h3m_final<SOLVER>, blocks(fbox), 256, 0, st, A, X);
+    chain(k_h3m_update, blocks(cells), 256, 0, st, A, X);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

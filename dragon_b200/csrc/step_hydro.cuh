@@ -9,6 +9,7 @@
 // set of Riemann pivots that can fail is the same.
 #pragma once
 
+#include "chain.cuh"
 #include "grid.cuh"
 #include "recon.cuh"
 #include "riemann.cuh"
@@ -98,6 +99,7 @@ template <int SOLVER, int TI, int TJ, int NT>
 __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
 k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa,
                const __grid_constant__ CUtensorMap tile_map) {
+    chained();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem2DH<TI, TJ>& S = *reinterpret_cast<Smem2DH<TI, TJ>*>(smem_raw);
     __shared__ int s_skip;
@@ -409,6 +411,7 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
 template <bool MHD, int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT)
 k_step1d(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+    chained();
     step1d_tile<MHD, SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }
 

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 
+#include "chain.cuh"
 #include "frame.cuh"
 #include "grid.cuh"
 #include "recon.cuh"
@@ -509,6 +510,7 @@ __device__ __forceinline__ void mhd2d_copy_frame(const Geo& G, const Geo& FG, co
 // Two CTAs per SM here too (160 registers unbounded: Orszag-Tang 384^2 0.153
 // ms a step, bounded 0.145).
 static __global__ void __launch_bounds__(256, 2) k_mhd2d_halfstates(Mhd2DArgs A) {
+    chained();
     const long long nthr = (long long)gridDim.x * gridDim.y * blockDim.x * blockDim.y;
     const long long tid = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * (blockDim.x * blockDim.y) +
                           threadIdx.y * blockDim.x + threadIdx.x;
@@ -518,13 +520,31 @@ static __global__ void __launch_bounds__(256, 2) k_mhd2d_halfstates(Mhd2DArgs A)
 // The flux kernels carry two CTAs per SM (<= 128 registers): at their natural
 // ~166 registers one 256-thread CTA fits, and the HLLD chains stall on latency.
 template <int SOLVER>
-__global__ void __launch_bounds__(256, 2) k_mhd2d_prelim(Mhd2DArgs A) { mhd2d_prelim<SOLVER>(A, launch_tile()); }
-static __global__ void k_mhd2d_e0(Mhd2DArgs A) { mhd2d_e0(A, launch_tile()); }
-static __global__ void __launch_bounds__(256, 2) k_mhd2d_half(Mhd2DArgs A) { mhd2d_half(A, launch_tile()); }
+__global__ void __launch_bounds__(256, 2) k_mhd2d_prelim(Mhd2DArgs A) {
+    chained();
+    mhd2d_prelim<SOLVER>(A, launch_tile());
+}
+static __global__ void k_mhd2d_e0(Mhd2DArgs A) {
+    chained();
+    mhd2d_e0(A, launch_tile());
+}
+static __global__ void __launch_bounds__(256, 2) k_mhd2d_half(Mhd2DArgs A) {
+    chained();
+    mhd2d_half(A, launch_tile());
+}
 template <int SOLVER>
-__global__ void __launch_bounds__(256, 2) k_mhd2d_final_flux(Mhd2DArgs A) { mhd2d_final_flux<SOLVER>(A, launch_tile()); }
-static __global__ void k_mhd2d_efinal(Mhd2DArgs A) { mhd2d_efinal(A, launch_tile()); }
-static __global__ void k_mhd2d_update(Mhd2DArgs A) { mhd2d_update(A, launch_tile()); }
+__global__ void __launch_bounds__(256, 2) k_mhd2d_final_flux(Mhd2DArgs A) {
+    chained();
+    mhd2d_final_flux<SOLVER>(A, launch_tile());
+}
+static __global__ void k_mhd2d_efinal(Mhd2DArgs A) {
+    chained();
+    mhd2d_efinal(A, launch_tile());
+}
+static __global__ void k_mhd2d_update(Mhd2DArgs A) {
+    chained();
+    mhd2d_update(A, launch_tile());
+}
 
 // 2D MHD CTU + CT step: the seven kernels in order; the first also copies
 // the ghost frame of the output buffers from the inputs (mhd2d_copy_frame).
@@ -535,13 +555,13 @@ inline int launch_step2d_mhd_t(const Geo& G, const Geo& FG, const double* w, dou
     const dim3 blk(kTileJ, kTileI);
     auto grid_for = [&](int ni, int nj) { return dim3((nj + kTileJ - 1) / kTileJ, (ni + kTileI - 1) / kTileI); };
     const int nx = G.n[0], ny = G.n[1];
-    k_mhd2d_halfstates<<<grid_for(nx + 4, ny + 4), blk, 0, st>>>(A);
-    k_mhd2d_prelim<SOLVER><<<grid_for(nx + 4, ny + 4), blk, 0, st>>>(A);
-    k_mhd2d_e0<<<grid_for(nx + 3, ny + 3), blk, 0, st>>>(A);
-    k_mhd2d_half<<<grid_for(nx + 2, ny + 2), blk, 0, st>>>(A);
-    k_mhd2d_final_flux<SOLVER><<<grid_for(nx + 2, ny + 2), blk, 0, st>>>(A);
-    k_mhd2d_efinal<<<grid_for(nx + 1, ny + 1), blk, 0, st>>>(A);
-    k_mhd2d_update<<<grid_for(nx, ny), blk, 0, st>>>(A);
+    chain(k_mhd2d_halfstates, grid_for(nx + 4, ny + 4), blk, 0, st, A);
+    chain(k_mhd2d_prelim<SOLVER>, grid_for(nx + 4, ny + 4), blk, 0, st, A);
+    chain(k_mhd2d_e0, grid_for(nx + 3, ny + 3), blk, 0, st, A);
+    chain(k_mhd2d_half, grid_for(nx + 2, ny + 2), blk, 0, st, A);
+    chain(k_mhd2d_final_flux<SOLVER>, grid_for(nx + 2, ny + 2), blk, 0, st, A);
+    chain(k_mhd2d_efinal, grid_for(nx + 1, ny + 1), blk, 0, st, A);
+    chain(k_mhd2d_update, grid_for(nx, ny), blk, 0, st, A);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

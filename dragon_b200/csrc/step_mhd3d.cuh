@@ -18,6 +18,7 @@
 // Every sweep covers the reference's index range, in its operand order.
 #pragma once
 
+#include "chain.cuh"
 #include "step3d.cuh"
 #include "step_mhd.cuh"
 
@@ -71,8 +72,13 @@ __device__ __forceinline__ bool m3_cell(long long t, int lo, int hi_incl, const 
 // Two CTAs per SM: natural register use (132; 196 for k_m3_half) leaves one,
 // and the capped builds measured 5 % faster on the 3D MHD step.
 static __global__ void __launch_bounds__(256, 2) k_m3_halfstates(Mhd3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
+    copy_shell<8>(A.G, shell_box(A.G, A.G.n, A.G.g, A.G.g), A.w, A.wout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
+    copy_shell<3>(A.FG, shell_box(A.FG, A.G.n, A.G.g, A.G.g + 1), A.B, A.Bout, blockIdx.x * blockDim.x + threadIdx.x,
+                  gridDim.x * blockDim.x);
     int i, j, k;
     if (!m3_cell(blockIdx.x * (long long)blockDim.x + threadIdx.x, -2, 1, A.G, i, j, k)) return;
     const double dt = *(const volatile double*)&A.ctl->t1;
@@ -137,6 +143,7 @@ __device__ __forceinline__ void m3_face_flux(const Mhd3DArgs& A, int i, int j, i
 // lower bound (-1 predictor, 0 final) up to the box's top.
 template <int SOLVER, bool FINAL>
 __global__ void __launch_bounds__(256, 2) k_m3_fluxes(Mhd3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -190,6 +197,7 @@ __device__ __forceinline__ V3 m3_edge_e(const Mhd3DArgs& A, const double* __rest
 // unbounded; both together 1.5 % of the 96^3 step).
 template <bool FINAL>
 __global__ void __launch_bounds__(256, 4) k_m3_edges(Mhd3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -224,6 +232,7 @@ struct M3Axis {
 
 // K4
 static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
+    chained();
     __shared__ int s;
     if (h3_skip(A.ctl, &s)) return;
     int i, j, k;
@@ -301,6 +310,7 @@ static __global__ void __launch_bounds__(256, 2) k_m3_half(Mhd3DArgs A) {
 
 // K7
 static __global__ void __launch_bounds__(256, 2) k_m3_update(Mhd3DArgs A) {
+    chained();
     __shared__ int s;
     __shared__ double red[32];
     if (h3_skip(A.ctl, &s)) return;
@@ -345,15 +355,13 @@ inline int launch_step3d_mhd_t(const Geo& G, const Geo& FG, const double* w, dou
         const long long n = (long long)(G.n[0] + hi - lo + 1) * (G.n[1] + hi - lo + 1) * (G.n[2] + hi - lo + 1);
         return (int)((n + 255) / 256);
     };
-    if (cudaMemcpyAsync(wout, w, sizeof(double) * 8 * G.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    if (cudaMemcpyAsync(Bout, B, sizeof(double) * 3 * FG.plane, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return 1;
-    k_m3_halfstates<<<blocks(-2, 1), 256, 0, st>>>(A);
-    k_m3_fluxes<SOLVER, false><<<blocks(-2, 1), 256, 0, st>>>(A);
-    k_m3_edges<false><<<blocks(-1, 1), 256, 0, st>>>(A);
-    k_m3_half<<<blocks(-1, 0), 256, 0, st>>>(A);
-    k_m3_fluxes<SOLVER, true><<<blocks(-1, 0), 256, 0, st>>>(A);
-    k_m3_edges<true><<<blocks(0, 0), 256, 0, st>>>(A);
-    k_m3_update<<<blocks(0, -1), 256, 0, st>>>(A);
+    chain(k_m3_halfstates, blocks(-2, 1), 256, 0, st, A);
+    chain(k_m3_fluxes<SOLVER, false>, blocks(-2, 1), 256, 0, st, A);
+    chain(k_m3_edges<false>, blocks(-1, 1), 256, 0, st, A);
+    chain(k_m3_half, blocks(-1, 0), 256, 0, st, A);
+    chain(k_m3_fluxes<SOLVER, true>, blocks(-1, 0), 256, 0, st, A);
+    chain(k_m3_edges<true>, blocks(0, 0), 256, 0, st, A);
+    chain(k_m3_update, blocks(0, -1), 256, 0, st, A);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

@@ -31,6 +31,7 @@
 // bounds clip each phase's rows and columns to those ranges at the grid edges.
 #pragma once
 
+#include "chain.cuh"
 #include "step_mhd_mixed.cuh"
 
 namespace dgpu {
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(NT, 2) k_mhd2d_fused_mixed(Geo G, Geo FG, cons
                                                           double* __restrict__ wout, const double* __restrict__ B,
                                                           double* __restrict__ Bout, StepCtl* ctl, StepArgs sa,
                                                           int seg_rows) {
+    chained();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& S = *reinterpret_cast<FusedMhdSmem<TJ, R>*>(smem_raw);
     mhd2d_fused_body<SOLVER, TJ, R, NT>(G, FG, w, wout, B, Bout, ctl, sa, seg_rows, blockIdx.x, blockIdx.y,

@@ -4,6 +4,7 @@
 // and fast single-precision division / square root.
 #include <algorithm>
 
+#include "chain.cuh"
 #include "launchers.h"
 #include "step_mhd_fused.cuh"
 
@@ -35,7 +36,7 @@ int launch_fused(const Geo& G, const Geo& FG, const double* w, double* wout, con
     int seg = (nx + segs_wanted - 1) / segs_wanted;
     seg = std::max(4 * kFuseR, (seg + kFuseR - 1) / kFuseR * kFuseR);
     const dim3 grid(strips, (nx + seg - 1) / seg);
-    kern<<<grid, kFuseNT, smem, st>>>(G, FG, w, wout, B, Bout, ctl, sa, seg);
+    chain(kern, grid, kFuseNT, smem, st, G, FG, w, wout, B, Bout, ctl, sa, seg);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

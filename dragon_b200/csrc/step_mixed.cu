@@ -14,6 +14,7 @@
 // double-precision arithmetic.
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "launchers.h"
 #include "mixed.cuh"
 #include "step_hydro.cuh"
@@ -74,6 +75,7 @@ template <int SOLVER, int TI, int TJ, int NT>
 __global__ void __launch_bounds__(NT, NT >= 384 ? 2 : 3)
 k_step2d_hydro_mixed(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa,
                      const __grid_constant__ CUtensorMap tile_map) {
+    chained();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SmemMixed<TI, TJ>& S = *reinterpret_cast<SmemMixed<TI, TJ>*>(smem_raw);
     __shared__ int s_skip;
@@ -280,7 +282,7 @@ static int launch_mixed_t(const Geo& G, const double* win, double* wout, StepCtl
         attr = true;
     }
     dim3 grid((G.n[1] + kMxTJ - 1) / kMxTJ, (G.n[0] + kMxTI - 1) / kMxTI);
-    kern<<<grid, kMxNT, smem, st>>>(G, win, wout, ctl, sa, *map);
+    chain(kern, grid, kMxNT, smem, st, G, win, wout, ctl, sa, *map);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
