@@ -51,7 +51,9 @@ namespace f64 {
 // to zero. A quotient that is a velocity, a field or a flux component raises
 // the flag when its numerator is smaller (quots); one that is only added to
 // something of normal size, which it then cannot change, passes as it is
-// (quotn).
+// (quot). A numerator that is infinite, NaN or too large needs no test of its
+// own there: it makes the quotient NaN or huge, and the sum, pressure, energy
+// or radicand it goes into has a test.
 
 // The flag of one face, cell or state. With LOCAL the quotients of small
 // numerators are divided by the plain operator on the spot: a branch per group
@@ -66,6 +68,10 @@ struct Flag {
     __device__ __forceinline__ void den(double x) {
         const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
         bad |= u - ((1023u - 120u) << 20) >= (170u << 20);
+    }
+    // x in [2^-120, 2^50)
+    __device__ __forceinline__ void posden(double x) {
+        bad |= (unsigned)__double2hiint(x) - ((1023u - 120u) << 20) >= (170u << 20);
     }
     // x in [2^-400, 2^400)
     __device__ __forceinline__ void pos(double x) {
@@ -120,58 +126,63 @@ __device__ __forceinline__ Rec rec(double b, C& ck) {
     ck.den(b);
     return rec_of(b);
 }
+// of a divisor that is positive (anything else raises the flag)
+struct PosRec : Rec {};
+template <class C>
+__device__ __forceinline__ PosRec posrec(double b, C& ck) {
+    ck.posden(b);
+    return PosRec{rec_of(b)};
+}
 
 // The sign a zero quotient takes (the corrections lose it); others have it already.
 __device__ __forceinline__ double signed_as(double q, double a, double b) {
     return __hiloint2double(__double2hiint(q) | ((__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000),
                             __double2loint(q));
 }
+__device__ __forceinline__ double signed_as(double q, double a, const Rec& r) { return signed_as(q, a, r.b); }
+__device__ __forceinline__ double signed_as(double q, double a, const PosRec&) {
+    return __hiloint2double(__double2hiint(q) | (__double2hiint(a) & (int)0x80000000), __double2loint(q));
+}
 
 // a / r.b, the numerator checked by the caller or known to be in range: the
-// quotient from both parts of the reciprocal, corrected once by its remainder.
+// quotient from both parts of the reciprocal, corrected once by its remainder
+// (a zero without its sign: for values that are not zero, or then added to one
+// that is not).
 __device__ __forceinline__ double quot(double a, const Rec& r) {
-    double q = __fma_rn(a, r.y, __dmul_rn(a, r.l));
+    const double q = __fma_rn(a, r.y, __dmul_rn(a, r.l));
     const double m = __fma_rn(-r.b, q, a);
-    q = __fma_rn(m, r.y, q);
-    return signed_as(q, a, r.b);
-}
-// a / r.b of a value that a small quotient cannot change.
-template <class C>
-__device__ __forceinline__ double quotn(double a, const Rec& r, C& ck) {
-    ck.fin(a);
-    return quot(a, r);
+    return __fma_rn(m, r.y, q);
 }
 // a / r.b for several values at once.
-template <class C, class... D>
-__device__ __forceinline__ void quots(const Rec& r, C& ck, D&... a) {
+template <class Q, class C, class... D>
+__device__ __forceinline__ void quots(const Q& r, C& ck, D&... a) {
     if constexpr (C::kLocal) {
         (ck.fin(a), ...);
         const bool small = (tiny(a) || ...);
         const double n[sizeof...(D)] = {a...};
-        ((a = quot(a, r)), ...);
+        ((a = signed_as(quot(a, r), a, r)), ...);
         if (small) {
             int k = 0;
             ((a = div_plain(n[k++], r.b)), ...);
         }
     } else {
         (ck.num(a), ...);
-        ((a = quot(a, r)), ...);
+        ((a = signed_as(quot(a, r), a, r)), ...);
     }
 }
 // a / b, one quotient (the first correction takes the place of the second
-// part of the reciprocal), without a look at the ranges
+// part of the reciprocal), without a look at the ranges or a zero's sign
 __device__ __forceinline__ double div_of(double a, double b) {
     const double y = reciprocal(b);
     double q = __dmul_rn(a, y);
     q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return signed_as(q, a, b);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 template <class C>
 __device__ __forceinline__ double div(double a, double b, C& ck) {
     ck.num(a);
     ck.den(b);
-    return div_of(a, b);
+    return signed_as(div_of(a, b), a, b);
 }
 
 __device__ __forceinline__ double root_of(double a) {
@@ -239,12 +250,12 @@ __device__ __forceinline__ Cons<double> to_cons(const Prim<double>& w) {
 template <bool MHD, class C>
 __device__ __forceinline__ double pressure(const Cons<double>& u, const Rec& r, C& ck) {
     ck.pos(u.E);
-    double Eth = u.E - 0.5 * quotn(dot3(u.mx, u.my, u.mz, u.mx, u.my, u.mz), r, ck);
+    double Eth = u.E - 0.5 * quot(dot3(u.mx, u.my, u.mz, u.mx, u.my, u.mz), r);
     if constexpr (MHD) Eth -= dot3(u.Bx, u.By, u.Bz, u.Bx, u.By, u.Bz) * k1_8pi;
     return kGm1 * Eth;
 }
 template <bool MHD, class C>
-__device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const Rec& r, C& ck) {
+__device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const PosRec& r, C& ck) {
     Prim<double> w;
     w.rho = u.rho;
     w.vx = u.mx;
@@ -257,10 +268,9 @@ __device__ __forceinline__ Prim<double> to_prim(const Cons<double>& u, const Rec
     return w;
 }
 // The flag unless is_physical holds for a state that to_prim gave without
-// one (its velocities are finite then).
+// one (its density is positive and its velocities are finite then).
 template <bool MHD, class C>
 __device__ __forceinline__ void sound_state(const Prim<double>& w, C& ck) {
-    ck.pos(w.rho);
     ck.pos(w.p);
     if constexpr (MHD) {
         ck.fin(w.Bx);
@@ -279,7 +289,7 @@ __device__ __forceinline__ Prim<double> corrected(const Prim<double>& w, const C
     Flag<LOCAL> ck;
     ck.pos(w.p);
     const Cons<double> u = c_sub<MHD>(f64::to_cons<MHD>(w), d);
-    Prim<double> r = f64::to_prim<MHD>(u, rec(u.rho, ck), ck);
+    Prim<double> r = f64::to_prim<MHD>(u, posrec(u.rho, ck), ck);
     if (ck.bad) {
         Prim<double> t = w;
         const Cons<double> e = d;
@@ -310,11 +320,14 @@ __device__ __forceinline__ Widths widths(int dim, double dx, double dy, double d
 template <class C>
 __device__ __forceinline__ double cfl_speed(const Prim<double>& w, double a, int cfl, const Widths& d, C& ck) {
     ck.raise(d.bad || cfl > 1);
-    double s = quotn(fabs(w.vx) + a, d.x, ck);
-    const double t = quotn(fabs(w.vy) + a, d.y, ck);
+    ck.fin(w.vx);
+    ck.fin(w.vy);
+    ck.fin(w.vz);
+    double s = quot(fabs(w.vx) + a, d.x);
+    const double t = quot(fabs(w.vy) + a, d.y);
     s = cfl == 0 ? smax(s, t) : s + t;
     if (d.three) {
-        const double t = quotn(fabs(w.vz) + a, d.z, ck);
+        const double t = quot(fabs(w.vz) + a, d.z);
         s = cfl == 0 ? smax(s, t) : s + t;
     }
     return s;
@@ -357,8 +370,8 @@ __device__ __forceinline__ double sound_speed(const Prim<double>& w, const Rec& 
 template <class C>
 __device__ __forceinline__ double fast_speed(const Prim<double>& w, double Bk, const Rec& r, C& ck) {
     const double c = f64::sound_speed(w, r, ck);
-    const double a = by_sq4pi(root0(quotn(dot3(w.Bx, w.By, w.Bz, w.Bx, w.By, w.Bz), r, ck), ck));
-    const double c2 = c * c, a2 = a * a, ak2 = quotn(Bk * Bk, r, ck) * k1_4pi;
+    const double a = by_sq4pi(root0(quot(dot3(w.Bx, w.By, w.Bz, w.Bx, w.By, w.Bz), r), ck));
+    const double c2 = c * c, a2 = a * a, ak2 = quot(Bk * Bk, r) * k1_4pi;
     const double s = c2 + a2;
     const double disc = smax(0.0, (s * s) * 0.25 - ak2 * c2);
     return root((c2 + a2) * 0.5 + root0(disc, ck), ck);
@@ -380,11 +393,9 @@ __device__ __forceinline__ void surely_physical(const Cons<double>& u, C& ck) {
     const double m2 = dot3(u.mx, u.my, u.mz, u.mx, u.my, u.mz);
     ck.pos(u.rho);
     ck.pos(u.E);
-    ck.fin(m2);
     double e = u.E * (1.0 - 0x1p-44);
     if constexpr (MHD) {
         const double b2 = dot3(u.Bx, u.By, u.Bz, u.Bx, u.By, u.Bz);
-        ck.fin(b2);
         e -= b2 * k1_8pi;
     }
     ck.raise(!(e * (2.0 * u.rho) > m2));

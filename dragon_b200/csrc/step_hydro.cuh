@@ -409,7 +409,7 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
 }
 
 template <bool MHD, int SOLVER, int TS, int NT>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 512 / NT)
 k_step1d(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
     chained();
     step1d_tile<MHD, SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);

@@ -147,7 +147,7 @@ __device__ __forceinline__ MhdCell mhd_cell(const Prim<double>& w, const StepArg
     ck.pos(w.p);
     Cons<double> U = f64::to_cons<true>(w);
     ((U = c_add<true>(U, d)), ...);
-    const Rec r = rec(U.rho, ck);
+    const PosRec r = posrec(U.rho, ck);
     ck.fin(U.E);
     ck.fin(U.Bx);
     ck.fin(U.By);

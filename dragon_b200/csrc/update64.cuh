@@ -32,7 +32,7 @@ __device__ __forceinline__ Updated updated(const Prim<double>& w, const StepArgs
     ck.pos(w.p);
     Cons<double> U = f64::to_cons<MHD>(w);
     ((U = c_add<MHD>(U, d)), ...);
-    const Rec r = rec(U.rho, ck);
+    const PosRec r = posrec(U.rho, ck);
     Updated o;
     o.w = f64::to_prim<MHD>(U, r, ck);
     sound_state<MHD>(o.w, ck);
