@@ -5,15 +5,14 @@
 
 namespace dgpu {
 
-// Tiles of 14 x 26 cells, 256 threads, two CTAs per SM (128 registers, 106 KB
+// Tiles of 16 x 24 cells, 256 threads, two CTAs per SM (128 registers, 111 KB
 // each): bound by FP64 issue, so one CTA's barriers, tile load and last rounds
 // of a phase fall under the other's arithmetic. Step time on the 1024^2 shear
-// layer, results bit-identical: 0.288 ms against 0.333 ms for one CTA of 19 x
-// 22 cells on 512 threads (the better shape while the divisions branched:
-// 0.471 against 0.51), 0.312 for 8 x 32, 0.296 for 12 x 30, 0.30 for 16 x 24
-// and 0.33 for three CTAs of 10 x 24 cells on 160 threads; x and y items in
-// one instruction sequence with a runtime direction 0.294.
-constexpr int k2dTI = 14, k2dTJ = 26, k2dNT = 256;
+// layer, results bit-identical: 0.256 ms (14 x 26 cells 0.261, 20 x 20 0.256, 18
+// x 22 0.263); one CTA of 28 x 30 cells on 512 threads 0.268, three of 10 x 24
+// on 160 threads 0.302, four of 8 x 22 on 128 threads 0.315. With divisions that
+// branched, one CTA of 19 x 22 cells on 512 threads was the best at 0.471.
+constexpr int k2dTI = 16, k2dTJ = 24, k2dNT = 256;
 
 // A grid whose large tiles do not fill the GPU waits for the longest CTA, not
 // for its arithmetic, so smaller grids take smaller tiles: 6 x 30 cells, whose
@@ -23,12 +22,12 @@ constexpr int k2dTI = 14, k2dTJ = 26, k2dNT = 256;
 // 26 cells: 96^2 22.6 / 24.7 / 32.9, 128^2 25.6 / 25.7 / 33.9, 200^2 35.6 / 31.0
 // / 33.1, 320^2 61.6 / 51.1 / 56.2, 400^2 85 / 68.5 / 68.6, 512^2 128 / 96 / 82.
 // Hence the lines: 6 x 14 up to one CTA per SM, 6 x 30 up to five.
-enum Tile2D { kTile14x26, kTile6x30, kTile6x14 };
+enum Tile2D { kTile16x24, kTile6x30, kTile6x14 };
 static Tile2D pick_tile(const Geo& G) {
     auto ctas = [&](int ti, int tj) { return (long long)((G.n[0] + ti - 1) / ti) * ((G.n[1] + tj - 1) / tj); };
     if (ctas(6, 14) <= 148) return kTile6x14;
     if (ctas(6, 30) <= 148 * 5) return kTile6x30;
-    return kTile14x26;
+    return kTile16x24;
 }
 
 template <int S, int TI, int TJ>
@@ -58,7 +57,7 @@ static int go(const Geo& G, const double* win, double* wout, StepCtl* ctl, const
 int step2d_tile_box(int mixed, const Geo& G, int box[3]) {
     const Tile2D t = pick_tile(G);
     box[0] = (mixed ? kMx2dTJ : t == kTile6x14 ? 14 : t == kTile6x30 ? 30 : k2dTJ) + 6;
-    box[1] = (mixed ? kMx2dTI : t == kTile14x26 ? k2dTI : 6) + 4;
+    box[1] = (mixed ? kMx2dTI : t == kTile16x24 ? k2dTI : 6) + 4;
     box[2] = 5;
     return 0;
 }

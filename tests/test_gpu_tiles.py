@@ -1,4 +1,4 @@
-"""The three tiles of the FP64 2D hydro step (6 x 14, 6 x 30, 14 x 26 cells,
+"""The three tiles of the FP64 2D hydro step (6 x 14, 6 x 30, 16 x 24 cells,
 chosen by the grid's extents) at the sizes where one gives way to the next and
 at their remainders, against the C restatement of the reference, bit for bit."""
 import numpy as np
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 # (nx, ny): a cell or two, one tile and its neighbours, the last 6 x 14 grid
-# (148 tiles) and the first 6 x 30 one, the last 6 x 30 grid (740) and the first of 14 x 26
+# (148 tiles) and the first 6 x 30 one, the last 6 x 30 grid (740) and the first of 16 x 24
 @pytest.mark.parametrize("nx,ny", [(2, 3), (6, 14), (7, 15), (12, 13), (222, 56), (223, 56), (24, 518), (24, 519),
                                    (444, 300), (445, 300), (60, 2220), (61, 2221)])
 @pytest.mark.parametrize("walls", [False, True])
