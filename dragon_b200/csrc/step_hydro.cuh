@@ -30,7 +30,7 @@ struct Smem2DH {
             double fy[5][TI + 2][TJ + 1];
         } f;
     } u;
-    double red[32];
+    unsigned long long vmax;  // bits of the largest CFL speed
     unsigned long long stat[7];
     uint64_t bar;
 };
@@ -115,6 +115,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
     FaceStats st{0, 0, 0, 0, 0};
     int first_order = 0;
     if (threadIdx.x < 7) S.stat[threadIdx.x] = 0;
+    if (threadIdx.x == 7) S.vmax = 0;
 
     // P0: tile + two-cell halo of the primitive state, one TMA copy of the five
     // planes (padded rows i0-2+g .., columns from the even column at or
@@ -265,8 +266,8 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
     }
     copy_ghosts_2d<5>(G, win, wout, i0, j0, TI, TJ);
 
-    vmax = block_max(vmax, S.red);
-    if (threadIdx.x == 0) atomic_max_speed(&ctl->vmax[sa.slot_out], vmax);
+    for (int o = 16; o > 0; o >>= 1) vmax = speed_max(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    if ((threadIdx.x & 31) == 0) atomic_max_speed(&S.vmax, vmax);
     // statistics
     if (st.pivot_exact) atomicAdd(&S.stat[0], (unsigned long long)st.pivot_exact);
     if (st.newton_iters) atomicAdd(&S.stat[2], (unsigned long long)st.newton_iters);
@@ -276,6 +277,7 @@ k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout,
     if (st.cap_hits) atomicAdd(&S.stat[6], (unsigned long long)st.cap_hits);
     __syncthreads();
     if (threadIdx.x == 0) {
+        if (S.vmax) atomicMax(&ctl->vmax[sa.slot_out], S.vmax);
         if (S.stat[0]) atomicAdd(&ctl->pivots_exact, S.stat[0]);
         if (S.stat[2]) atomicAdd(&ctl->newton_iters, S.stat[2]);
         if (S.stat[3]) atomicAdd(&ctl->exact_calls, S.stat[3]);
