@@ -284,13 +284,11 @@ __device__ __forceinline__ Cons<double> roe(const Prim<double>& L, const Prim<do
 }
 
 // ---------------------------------------------------------------------------
-// The exact solver (Exact.cpp) with the reference's mean guess or the analytic
-// one. What bounds it is pow, so a power of one (a uniform or a resting gas,
-// both sides of most faces ahead of a front) is not taken, and the
-// derivative's power -(g + 1) / (2 g) is the function's (g - 1) / (2 g) divided
-// by the argument: it steers the Newton step alone, whose end the tolerance
-// sets. 3D blast 110 x 87 x 93, two steps: 5.77 ms from the start of the blast
-// and 7.97 over a long run with the plain solver, 2.80 and 6.88 with this one.
+// The exact solver (Exact.cpp) with the reference's mean guess. What bounds it
+// is pow, so a power of one (a uniform or a resting gas, both sides of most
+// faces ahead of a front) is not taken, and the derivative's power -(g + 1) /
+// (2 g) is the function's (g - 1) / (2 g) divided by the argument (their sum
+// is -1): it steers the Newton step alone, whose end the tolerance sets.
 
 __device__ __forceinline__ double pow1(double x, double y) { return x == 1.0 ? 1.0 : pow(x, y); }
 
@@ -327,9 +325,6 @@ __device__ __forceinline__ double exact_rho(double p, const Prim<double>& w, con
     if (p > w.p) return div(w.rho * (p + s.B), kGm1_Gp1 * p + w.p, ck);
     return w.rho * pow1(quot(p, s.rp), kGinv);
 }
-static __device__ __noinline__ double analytic_guess_of(const Prim<double>* LR) {
-    return dgpu::analytic_guess(LR[0], LR[1]);
-}
 // the flux of the exact solution at x / t = 0
 template <class C>
 __device__ __forceinline__ Cons<double> exact(const Prim<double>& L, const Prim<double>& Rt, const ExactOpts& o,
@@ -349,10 +344,6 @@ __device__ __forceinline__ Cons<double> exact(const Prim<double>& L, const Prim<
         rhoR = Rt.rho * pow1(quot(p, sR.rp), kGinv);
     } else {
         p = (L.p + Rt.p) * 0.5;
-        if (o.guess == GUESS_ANALYTIC) {
-            const Prim<double> LR[2] = {L, Rt};
-            p = analytic_guess_of(LR);
-        }
         double CHA;
         int iters = o.max_iters, n = 0;
         do {
@@ -663,7 +654,7 @@ __device__ __noinline__ bool face_slow(const Prim<double>* LR, double dt_dx, con
 
 // The flux along x of the states on both sides of a face, as face_flux_x. MHD
 // HLL is rare and takes the plain routine, and so does the exact solver with
-// the learned or the measured guess or while its solves are logged.
+// another guess than the mean or while its solves are logged.
 template <bool MHD, int SOLVER, bool LOCAL = false>
 __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
                                             const ExactOpts& eo, Cons<double>& F, FaceStats* st) {
@@ -673,7 +664,7 @@ __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<do
         constexpr bool kExact = !MHD && SOLVER == RS_EXACT;
         Flag<LOCAL> ck;
         FaceStats s = *st;
-        const bool plain = kExact && ((eo.guess != GUESS_MEAN && eo.guess != GUESS_ANALYTIC) || eo.log.rows);
+        const bool plain = kExact && (eo.guess != GUESS_MEAN || eo.log.rows);
         if (!plain) {
             face_body<MHD, SOLVER>(L, Rt, dt_dL, eo, F, &s, ck);
             if (!ck.bad) {
