@@ -48,7 +48,7 @@ struct PrologueArgs {
 // layer) by the calling threads: tid of nthreads (one CTA in the prologue, a
 // whole grid in k_bc_pass).
 template <bool MHD>
-__device__ void bc_cells_axis(const Geo& G, double* __restrict__ w, const BCEntry& e, int a, long long tid,
+__host__ __device__ inline void bc_cells_axis(const Geo& G, double* __restrict__ w, const BCEntry& e, int a, long long tid,
                               long long nthreads) {
     const int dim = G.dim, ng = G.g;
     const int na = G.n[a];
@@ -127,7 +127,7 @@ __device__ void bc_cells_axis(const Geo& G, double* __restrict__ w, const BCEntr
 // Face-B ghosts of one entry along one axis. FG is the face geometry (n+1 per
 // axis); n_cells the cell extents. One thread per (side, transverse point)
 // runs the sequential ghost-layer recurrence.
-__device__ inline void bc_faces_axis(const Geo& FG, const int* ncell, double* __restrict__ B, const BCEntry& e, int a,
+__host__ __device__ inline void bc_faces_axis(const Geo& FG, const int* ncell, double* __restrict__ B, const BCEntry& e, int a,
                                      long long tid, long long nthreads) {
     const int dim = FG.dim, ng = FG.g;
     const int na = ncell[a];
@@ -510,7 +510,8 @@ __global__ void __launch_bounds__(256) k_prologue_coop(Geo G, Geo FG, double* __
 // shear layer 1024^2 0.290 and 0.279 ms (mixed 0.167 and 0.157), Orszag-Tang
 // 384^2 0.176 and 0.158, 3D blast 128^3 2.20 and 2.16. It stays for lists with
 // corner ghosts off, with Reflective or Fixed faces of an MHD grid (their
-// face-B passes read what they wrote) and for extents below the ghost width.
+// face-B passes read what they wrote), with a Periodic over an Outflow face of
+// one (direct_fill_ok) and for extents below the ghost width.
 constexpr int kDirectEntries = 8;
 struct DirectList {
     int n;
@@ -518,22 +519,28 @@ struct DirectList {
 };
 
 // Whether the entries [first, first + count) of a list can be filled in one pass.
+// Of an MHD grid no Periodic entry may follow an Outflow on the same upper
+// face: Periodic leaves the outermost face point of that side alone, whose
+// Outflow value was extrapolated from the boundary face that Periodic then
+// writes, so a thread would read what another one writes.
 inline bool direct_fill_ok(const Geo& G, const BCEntry* e, int first, int count, bool mhd) {
     if (G.dim < 2 || count > kDirectEntries) return false;
     for (int a = 0; a < G.dim; a++)
         if (G.n[a] < G.g + 1) return false;
+    int out = 0;  // upper faces of the Outflow entries so far
     for (int k = first; k < first + count; k++) {
         if (e[k].type == BC_IGNORE) continue;
         if (!e[k].corners) return false;
         if (mhd && (e[k].type == BC_REFLECTIVE || e[k].type == BC_FIXED)) return false;
+        if (mhd && e[k].type == BC_PERIODIC && (e[k].faces & out)) return false;
+        if (e[k].type == BC_OUTFLOW || e[k].type == BC_OUTFLOW_GATED) out |= e[k].faces & (FX_POS | FY_POS | FZ_POS);
     }
     return true;
 }
 
 // The value of ghost cell c after every pass of the list; false if none writes it.
 template <bool MHD>
-__device__ __forceinline__ bool direct_cell(const Geo& G, const double* __restrict__ w, const DirectList& list,
-                                            const int* c, Prim<double>& v) {
+DHD bool direct_cell(const Geo& G, const double* __restrict__ w, const DirectList& list, const int* c, Prim<double>& v) {
     int q[3] = {c[0], c[1], c[2]};
     unsigned flip = 0, gate_lo = 0, gate_hi = 0;  // by axis
     int fixed = -1;
@@ -585,8 +592,8 @@ __device__ __forceinline__ bool direct_cell(const Geo& G, const double* __restri
 // Walks point q from pass `last` (3 entry + axis) down. Returns whether some
 // pass writes it; axis: the one an extrapolating pass stopped at (-1: none),
 // with the layers from the face and the pass to go on with.
-__device__ __forceinline__ bool direct_walk(const Geo& FG, const DirectList& list, const int* ncell, int comp, int last,
-                                            int* q, int& axis, int& steps, int& next) {
+DHD bool direct_walk(const Geo& FG, const DirectList& list, const int* ncell, int comp, int last, int* q, int& axis,
+                     int& steps, int& next) {
     bool hit = false;
     axis = -1;
     for (int e = last / 3; e >= 0 && axis < 0; e--) {
@@ -616,8 +623,8 @@ __device__ __forceinline__ bool direct_walk(const Geo& FG, const DirectList& lis
     }
     return hit;
 }
-__device__ __forceinline__ bool direct_face(const Geo& FG, const double* __restrict__ B, const DirectList& list,
-                                            const int* ncell, const int* p, int comp, double& v) {
+DHD bool direct_face(const Geo& FG, const double* __restrict__ B, const DirectList& list, const int* ncell, const int* p,
+                     int comp, double& v) {
     int q[3] = {p[0], p[1], p[2]}, axis, steps = 0, next = 0;
     const double* Bc = B + comp * FG.plane;
     if (!direct_walk(FG, list, ncell, comp, 3 * list.n - 1, q, axis, steps, next)) return false;

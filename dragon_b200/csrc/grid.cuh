@@ -29,11 +29,11 @@ struct Geo {
 };
 
 // Cell index (i,j,k) in interior coordinates (ghosts negative / >= n).
-__device__ __forceinline__ long long gidx1(const Geo& G, int i) { return (long long)(i + G.g); }
-__device__ __forceinline__ long long gidx2(const Geo& G, int i, int j) {
+DHD long long gidx1(const Geo& G, int i) { return (long long)(i + G.g); }
+DHD long long gidx2(const Geo& G, int i, int j) {
     return (long long)(i + G.g) * G.pitch + (j + G.g);
 }
-__device__ __forceinline__ long long gidx3(const Geo& G, int i, int j, int k) {
+DHD long long gidx3(const Geo& G, int i, int j, int k) {
     return (long long)(i + G.g) * G.pitch2 + (long long)(j + G.g) * G.pitch + (k + G.g);
 }
 
@@ -43,7 +43,7 @@ struct ShellBox {
     int n[3], lo, hi, dim;
     unsigned s0, s1, total;  // items of the first axis' slabs, of the first two
 };
-__host__ __device__ __forceinline__ ShellBox shell_box(const Geo& G, const int* n, int lo, int hi) {
+DHD ShellBox shell_box(const Geo& G, const int* n, int lo, int hi) {
     ShellBox b;
     b.dim = G.dim;
     b.lo = lo;
@@ -56,7 +56,7 @@ __host__ __device__ __forceinline__ ShellBox shell_box(const Geo& G, const int* 
     b.total = G.dim > 2 ? b.s1 + (unsigned)b.n[0] * b.n[1] * w : b.s1;
     return b;
 }
-__device__ __forceinline__ void shell_point(const ShellBox& b, unsigned t, int* c) {
+DHD void shell_point(const ShellBox& b, unsigned t, int* c) {
     const unsigned w = b.lo + b.hi;
     const unsigned e1 = b.n[1] + w, e2 = b.dim > 2 ? b.n[2] + w : 1;
     auto layer = [&](unsigned l, int n) { return (int)l < b.lo ? (int)l - b.lo : n + (int)l - b.lo; };
@@ -79,7 +79,7 @@ __device__ __forceinline__ void shell_point(const ShellBox& b, unsigned t, int* 
         c[1] = q % b.n[1];
     }
 }
-__device__ __forceinline__ long long gidx(const Geo& G, const int* c) {
+DHD long long gidx(const Geo& G, const int* c) {
     return G.dim == 2 ? gidx2(G, c[0], c[1]) : gidx3(G, c[0], c[1], c[2]);
 }
 
@@ -216,7 +216,7 @@ __device__ __forceinline__ double grid_cfl_speed(const Prim<double>& W, int dim,
 
 // Field-plane accessors.
 template <bool MHD>
-__device__ __forceinline__ Prim<double> load_prim(const double* __restrict__ w, long long plane, long long m) {
+DHD Prim<double> load_prim(const double* __restrict__ w, long long plane, long long m) {
     Prim<double> r;
     r.rho = w[m];
     r.p = w[plane + m];
@@ -233,7 +233,7 @@ __device__ __forceinline__ Prim<double> load_prim(const double* __restrict__ w, 
     return r;
 }
 template <bool MHD>
-__device__ __forceinline__ void store_prim(double* __restrict__ w, long long plane, long long m, const Prim<double>& r) {
+DHD void store_prim(double* __restrict__ w, long long plane, long long m, const Prim<double>& r) {
     w[m] = r.rho;
     w[plane + m] = r.p;
     w[2 * plane + m] = r.vx;
