@@ -15,6 +15,12 @@ namespace dgpu {
 // First statement of every thread of a kernel that chain() launches. No thread
 // may leave before it: the kernel after this one takes this one's end for the
 // end of all before it.
+//
+// What the kernel before it may write is read with plain loads, after this
+// statement, which no load is moved above. The read-only path (ld.global.nc:
+// __ldg, or a kernel parameter that is const and __restrict__) is for memory
+// that nobody writes from the reading kernel's launch on, and such a load may
+// be moved up. tests/test_chained_loads.py looks for both.
 __device__ __forceinline__ void chained() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

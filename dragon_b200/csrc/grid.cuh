@@ -93,8 +93,11 @@ __device__ __forceinline__ void copy_shell(const Geo& G, const ShellBox& b, cons
         int c[3];
         shell_point(b, t, c);
         const long long m = gidx(G, c);
+        double v[NF];  // all loads before the first store
 #pragma unroll
-        for (int f = 0; f < NF; f++) out[f * G.plane + m] = in[f * G.plane + m];
+        for (int f = 0; f < NF; f++) v[f] = in[f * G.plane + m];
+#pragma unroll
+        for (int f = 0; f < NF; f++) out[f * G.plane + m] = v[f];
     }
 }
 

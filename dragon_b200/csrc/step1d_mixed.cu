@@ -11,7 +11,7 @@ namespace {
 
 template <int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT)
-k_step1d_mx(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+k_step1d_mx(Geo G, const double* win, double* wout, StepCtl* ctl, StepArgs sa) {
     chained();
     step1d_tile_mx<SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }
@@ -20,7 +20,7 @@ k_step1d_mx(Geo G, const double* __restrict__ win, double* __restrict__ wout, St
 // FP32 fields in static shared memory), as the FP64 MHD sweep.
 template <int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT)
-k_step1d_mx_mhd(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+k_step1d_mx_mhd(Geo G, const double* win, double* wout, StepCtl* ctl, StepArgs sa) {
     chained();
     step1d_tile_mx_mhd<SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }

@@ -47,24 +47,21 @@ __device__ __forceinline__ bool box_cell(long long t, const int* lo, const int* 
     return true;
 }
 
-// Every array a kernel of this step reads is one it does not write (state ->
-// half states -> predictor fluxes -> corner fluxes -> final fluxes -> new
-// state), so the loads go through the read-only path: the compiler may then
-// issue a later face's loads before an earlier face's stores.
+// Plain loads: the kernel before this one may still write these arrays while
+// this one's CTAs wait (chain.cuh).
 __device__ __forceinline__ Prim<double> ld5(const double* a, long long P, long long m) {
     Prim<double> r;
-    r.rho = __ldg(a + m);
-    r.p = __ldg(a + P + m);
-    r.vx = __ldg(a + 2 * P + m);
-    r.vy = __ldg(a + 3 * P + m);
-    r.vz = __ldg(a + 4 * P + m);
+    r.rho = a[m];
+    r.p = a[P + m];
+    r.vx = a[2 * P + m];
+    r.vy = a[3 * P + m];
+    r.vz = a[4 * P + m];
     r.Bx = r.By = r.Bz = 0;
     return r;
 }
 __device__ __forceinline__ void st5(double* a, long long P, long long m, const Prim<double>& w) { store_prim<false>(a, P, m, w); }
 __device__ __forceinline__ Cons<double> ldc5(const double* a, long long P, long long m) {
-    return Cons<double>{__ldg(a + m), __ldg(a + P + m), __ldg(a + 2 * P + m), __ldg(a + 3 * P + m), __ldg(a + 4 * P + m),
-                        0, 0, 0};
+    return Cons<double>{a[m], a[P + m], a[2 * P + m], a[3 * P + m], a[4 * P + m], 0, 0, 0};
 }
 __device__ __forceinline__ void stc5(double* a, long long P, long long m, const Cons<double>& u) {
     a[m] = u.rho; a[P + m] = u.E; a[2 * P + m] = u.mx; a[3 * P + m] = u.my; a[4 * P + m] = u.mz;

@@ -36,11 +36,6 @@ __device__ __forceinline__ float* m3m_hs(const Mx3M& X, int axis, int side) {
 __device__ __forceinline__ float* m3m_flux(const Mx3M& X, int axis) { return axis == 0 ? X.fx : axis == 1 ? X.fy : X.fz; }
 
 __device__ __forceinline__ Prim<float> ldf8(const float* a, long long P, long long m) {
-    return Prim<float>{__ldg(a + m),         __ldg(a + P + m),     __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                       __ldg(a + 4 * P + m), __ldg(a + 5 * P + m), __ldg(a + 6 * P + m), __ldg(a + 7 * P + m)};
-}
-// plain loads: the half states k_m3m_half corrects in place
-__device__ __forceinline__ Prim<float> ldf8_rw(const float* a, long long P, long long m) {
     return Prim<float>{a[m], a[P + m], a[2 * P + m], a[3 * P + m], a[4 * P + m], a[5 * P + m], a[6 * P + m], a[7 * P + m]};
 }
 __device__ __forceinline__ void stf8(float* a, long long P, long long m, const Prim<float>& w) {
@@ -48,8 +43,7 @@ __device__ __forceinline__ void stf8(float* a, long long P, long long m, const P
     a[4 * P + m] = w.vz; a[5 * P + m] = w.Bx; a[6 * P + m] = w.By; a[7 * P + m] = w.Bz;
 }
 __device__ __forceinline__ Cons<float> ldcf8(const float* a, long long P, long long m) {
-    return Cons<float>{__ldg(a + m),         __ldg(a + P + m),     __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                       __ldg(a + 4 * P + m), __ldg(a + 5 * P + m), __ldg(a + 6 * P + m), __ldg(a + 7 * P + m)};
+    return Cons<float>{a[m], a[P + m], a[2 * P + m], a[3 * P + m], a[4 * P + m], a[5 * P + m], a[6 * P + m], a[7 * P + m]};
 }
 __device__ __forceinline__ void stcf8(float* a, long long P, long long m, const Cons<float>& u) {
     a[m] = u.rho; a[P + m] = u.E; a[2 * P + m] = u.mx; a[3 * P + m] = u.my;
@@ -155,9 +149,9 @@ __device__ __forceinline__ V3 m3m_edge_e(const Mhd3DArgs& A, const Mx3M& X, cons
                                          int j, int k) {
     const Geo& F = A.FG;
     const long long SP = X.plane;
-    auto Xf = [&](int a, int b, int c, int q) { return (double)__ldg(X.fx + q * SP + gidx3(F, a, b, c)); };
-    auto Yf = [&](int a, int b, int c, int q) { return (double)__ldg(X.fy + q * SP + gidx3(F, a, b, c)); };
-    auto Zf = [&](int a, int b, int c, int q) { return (double)__ldg(X.fz + q * SP + gidx3(F, a, b, c)); };
+    auto Xf = [&](int a, int b, int c, int q) { return (double)X.fx[q * SP + gidx3(F, a, b, c)]; };
+    auto Yf = [&](int a, int b, int c, int q) { return (double)X.fy[q * SP + gidx3(F, a, b, c)]; };
+    auto Zf = [&](int a, int b, int c, int q) { return (double)X.fz[q * SP + gidx3(F, a, b, c)]; };
     auto ER = [&](int a, int b, int c) { return m3_ld_v3(eref, SP, gidx3(F, a, b, c)); };
     // flux planes: 0 rho, 1 E, 2-4 momentum, 5 Bx, 6 By, 7 Bz
     V3 e;
@@ -236,7 +230,7 @@ __global__ void __launch_bounds__(256, 2) k_m3m_half(Mhd3DArgs A, Mx3M X) {
     auto apply = [&](int axis, Cons<float> corr, double bl, double br) {
         float* pl = m3m_hs(X, axis, 0);
         float* pr = m3m_hs(X, axis, 1);
-        const Prim<float> sL = ldf8_rw(pl, SP, m), sR = ldf8_rw(pr, SP, m);
+        const Prim<float> sL = ldf8(pl, SP, m), sR = ldf8(pr, SP, m);
         Cons<float> uL = c_add<true>(to_cons<true>(sL), corr);
         Cons<float> uR = c_add<true>(to_cons<true>(sR), corr);
         if (axis == 0) { uL.Bx = (float)bl; uR.Bx = (float)br; }
@@ -311,7 +305,7 @@ __global__ void __launch_bounds__(256) k_m3m_update(Mhd3DArgs A, Mx3M X) {
             const float* Fl = m3m_flux(X, ax);
 #pragma unroll
             for (int q = 0; q < 8; q++)
-                *u8[q] += ((double)__ldg(Fl + q * SP + mf) - (double)__ldg(Fl + q * SP + up[ax])) * d[ax];
+                *u8[q] += ((double)Fl[q * SP + mf] - (double)Fl[q * SP + up[ax]]) * d[ax];
         }
         if (!is_finite<true>(U)) record_error(A.ctl, ST_NAN, mc);
         Prim<double> nw = body_field(to_prim64<true>(U), (b.bx0 + b.bx1) * 0.5, (b.by0 + b.by1) * 0.5,

@@ -28,15 +28,13 @@ struct Mx3 {
 };
 
 __device__ __forceinline__ Prim<float> ldf5(const float* a, long long P, long long m) {
-    return Prim<float>{__ldg(a + m), __ldg(a + P + m), __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                       __ldg(a + 4 * P + m), 0.f, 0.f, 0.f};
+    return Prim<float>{a[m], a[P + m], a[2 * P + m], a[3 * P + m], a[4 * P + m], 0.f, 0.f, 0.f};
 }
 __device__ __forceinline__ void stf5(float* a, long long P, long long m, const Prim<float>& w) {
     a[m] = w.rho; a[P + m] = w.p; a[2 * P + m] = w.vx; a[3 * P + m] = w.vy; a[4 * P + m] = w.vz;
 }
 __device__ __forceinline__ Cons<float> ldcf5(const float* a, long long P, long long m) {
-    return Cons<float>{__ldg(a + m), __ldg(a + P + m), __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                       __ldg(a + 4 * P + m), 0.f, 0.f, 0.f};
+    return Cons<float>{a[m], a[P + m], a[2 * P + m], a[3 * P + m], a[4 * P + m], 0.f, 0.f, 0.f};
 }
 __device__ __forceinline__ void stcf5(float* a, long long P, long long m, const Cons<float>& u) {
     a[m] = u.rho; a[P + m] = u.E; a[2 * P + m] = u.mx; a[3 * P + m] = u.my; a[4 * P + m] = u.mz;
@@ -250,7 +248,7 @@ __global__ void __launch_bounds__(256) k_h3m_update(Step3DArgs A, Mx3 X) {
             const float* F = X.pf + 5 * ax * SP;
 #pragma unroll
             for (int f = 0; f < 5; f++)
-                *u5[f] += ((double)__ldg(F + f * SP + m) - (double)__ldg(F + f * SP + up[ax])) * d[ax];
+                *u5[f] += ((double)F[f * SP + m] - (double)F[f * SP + up[ax]]) * d[ax];
         }
         const Prim<double> nw = to_prim64<false>(U);
         if (!is_finite<false>(U)) record_error(A.ctl, ST_NAN, m);

@@ -90,14 +90,17 @@ __device__ __forceinline__ void copy_ghosts_2d(const Geo& G, const double* __res
         const int i = lo_i + t / wj, j = lo_j + t % wj;
         if (i >= 0 && i < nx && j >= 0 && j < ny) continue;
         const long long m = gidx2(G, i, j);
+        double v[NF];  // all loads before the first store
 #pragma unroll
-        for (int f = 0; f < NF; f++) wout[f * G.plane + m] = win[f * G.plane + m];
+        for (int f = 0; f < NF; f++) v[f] = win[f * G.plane + m];
+#pragma unroll
+        for (int f = 0; f < NF; f++) wout[f * G.plane + m] = v[f];
     }
 }
 
 template <int SOLVER, int TI, int TJ, int NT>
 __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
-k_step2d_hydro(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa,
+k_step2d_hydro(Geo G, const double* win, double* wout, StepCtl* ctl, StepArgs sa,
                const __grid_constant__ CUtensorMap tile_map) {
     chained();
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -412,7 +415,7 @@ __device__ __forceinline__ void step1d_tile(const Geo& G, const double* __restri
 
 template <bool MHD, int SOLVER, int TS, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
-k_step1d(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa) {
+k_step1d(Geo G, const double* win, double* wout, StepCtl* ctl, StepArgs sa) {
     chained();
     step1d_tile<MHD, SOLVER, TS>(G, win, wout, ctl, sa, blockIdx.x);
 }

@@ -480,8 +480,11 @@ __device__ __forceinline__ void mhd2d_copy_frame(const Geo& G, const Geo& FG, co
         if (k < nc) {
             if (!frame_point(k, -g, nx + g, -g, ny + g, 0, nx, 0, ny, i, j)) continue;
             const long long m = gidx2(G, i, j);
+            double v[8];  // all loads before the first store
 #pragma unroll
-            for (int f = 0; f < 8; f++) wout[f * G.plane + m] = w[f * G.plane + m];
+            for (int f = 0; f < 8; f++) v[f] = w[f * G.plane + m];
+#pragma unroll
+            for (int f = 0; f < 8; f++) wout[f * G.plane + m] = v[f];
             continue;
         }
         long long q = k - nc;

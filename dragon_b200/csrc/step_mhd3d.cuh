@@ -46,20 +46,19 @@ __device__ __forceinline__ double* m3_flux_w(const Mhd3DArgs& A, int axis) {
     return axis == 0 ? A.S.fx : axis == 1 ? A.S.fy : A.S.fz;
 }
 
-// Read-only loads (ld.global.nc). Every array these are used on is one the
-// calling kernel does not write; the half states that k_m3_half corrects in
-// place keep plain loads there.
-__device__ __forceinline__ double m3_ld(const double* a, long long m) { return __ldg(a + m); }
+// Plain loads: the kernel before this one may still write these arrays while
+// this one's CTAs wait (chain.cuh).
+__device__ __forceinline__ double m3_ld(const double* a, long long m) { return a[m]; }
 __device__ __forceinline__ Prim<double> m3_ld_prim(const double* a, long long P, long long m) {
-    return Prim<double>{__ldg(a + m),         __ldg(a + P + m),     __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                        __ldg(a + 4 * P + m), __ldg(a + 5 * P + m), __ldg(a + 6 * P + m), __ldg(a + 7 * P + m)};
+    return Prim<double>{a[m],         a[P + m],     a[2 * P + m], a[3 * P + m],
+                        a[4 * P + m], a[5 * P + m], a[6 * P + m], a[7 * P + m]};
 }
 __device__ __forceinline__ Cons<double> m3_ld_cons(const double* a, long long P, long long m) {
-    return Cons<double>{__ldg(a + m),         __ldg(a + P + m),     __ldg(a + 2 * P + m), __ldg(a + 3 * P + m),
-                        __ldg(a + 4 * P + m), __ldg(a + 5 * P + m), __ldg(a + 6 * P + m), __ldg(a + 7 * P + m)};
+    return Cons<double>{a[m],         a[P + m],     a[2 * P + m], a[3 * P + m],
+                        a[4 * P + m], a[5 * P + m], a[6 * P + m], a[7 * P + m]};
 }
 __device__ __forceinline__ V3 m3_ld_v3(const double* a, long long P, long long m) {
-    return V3{__ldg(a + m), __ldg(a + P + m), __ldg(a + 2 * P + m)};
+    return V3{a[m], a[P + m], a[2 * P + m]};
 }
 
 __device__ __forceinline__ bool m3_cell(long long t, int lo, int hi_incl, const Geo& G, int& i, int& j, int& k) {

@@ -430,10 +430,8 @@ __device__ __forceinline__ void mhd2d_fused_body(const Geo& G, const Geo& FG, co
 
 // The single-grid step: a strip per blockIdx.x, a segment per blockIdx.y.
 template <int SOLVER, int TJ, int R, int NT>
-__global__ void __launch_bounds__(NT, 2) k_mhd2d_fused_mixed(Geo G, Geo FG, const double* __restrict__ w,
-                                                          double* __restrict__ wout, const double* __restrict__ B,
-                                                          double* __restrict__ Bout, StepCtl* ctl, StepArgs sa,
-                                                          int seg_rows) {
+__global__ void __launch_bounds__(NT, 2) k_mhd2d_fused_mixed(Geo G, Geo FG, const double* w, double* wout, const double* B,
+                                                          double* Bout, StepCtl* ctl, StepArgs sa, int seg_rows) {
     chained();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& S = *reinterpret_cast<FusedMhdSmem<TJ, R>*>(smem_raw);

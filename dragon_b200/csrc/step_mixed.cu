@@ -73,7 +73,7 @@ __device__ __forceinline__ double block_min(double v, double* scratch) {
 // faster than two CTAs at 110 registers on a 2048^2 shear layer, same results.
 template <int SOLVER, int TI, int TJ, int NT>
 __global__ void __launch_bounds__(NT, NT >= 384 ? 2 : 3)
-k_step2d_hydro_mixed(Geo G, const double* __restrict__ win, double* __restrict__ wout, StepCtl* ctl, StepArgs sa,
+k_step2d_hydro_mixed(Geo G, const double* win, double* wout, StepCtl* ctl, StepArgs sa,
                      const __grid_constant__ CUtensorMap tile_map) {
     chained();
     extern __shared__ __align__(128) unsigned char smem_raw[];
