@@ -362,7 +362,10 @@ int retry_member(dragon_grid* h, int* retries) {
         if (!C.err) break;
     }
     C.cur = c ^ 1;  // the retried step is committed; the next prologue accounts it
-    return push_ctl(h);
+    if ((rc = push_ctl(h))) return rc;
+    // the batch's stream reads the block next, and this mirror is written again
+    CKB(cudaStreamSynchronize(h->stream));
+    return 0;
 }
 
 int advance(dragon_batch* b, int nsteps, dragon_batch_stats* st) {
@@ -370,7 +373,9 @@ int advance(dragon_batch* b, int nsteps, dragon_batch_stats* st) {
     const int n = (int)b->members.size();
     if (n == 0 || nsteps == 0) return 0;
     int rc;
-    // members' pending work, then each member's control block for this advance
+    // members' pending work (a copy from hctl may be among it), then each
+    // member's control block for this advance
+    for (dragon_grid* h : b->members) CKB(cudaStreamSynchronize(h->stream));
     if (b->dirty && (rc = build(b))) return rc;
     for (int i = 0; i < n; i++) {
         dragon_grid* h = b->members[i];
@@ -382,7 +387,8 @@ int advance(dragon_batch* b, int nsteps, dragon_batch_stats* st) {
         h->hctl->cur = h->cur;
         b->h_all[i] = *h->hctl;
     }
-    for (dragon_grid* h : b->members) CKB(cudaStreamSynchronize(h->stream));
+    for (dragon_grid* h : b->members)
+        if (!h->imax_valid) CKB(cudaStreamSynchronize(h->stream));
     CKB(cudaMemcpyAsync(b->d_all, b->h_all, sizeof(StepCtl) * n, cudaMemcpyHostToDevice, b->stream));
     k_batch_ctl<true><<<(n * 32 + 255) / 256, 256, 0, b->stream>>>(b->d_insts, n, b->d_all);
     CKB(cudaGetLastError());
