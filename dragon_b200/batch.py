@@ -26,7 +26,7 @@ class Tuning:
     ctas_per_sm: int = 0     # 0: as many as fit
     order: int = ORDER_PHASE_MAJOR
     graph_steps: int = 32
-    mhd_tiles: int = 8       # 32 x 8 tiles of a 2D MHD phase per work item
+    mhd_tiles: int = 8       # 32 x 8 tiles of a 2D MHD phase per work item (an untuned batch: up to 8)
     wave: int = 1            # ORDER_WAVEFRONT: 2D MHD grids per wavefront group
 
     def to_c(self):

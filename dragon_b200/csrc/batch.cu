@@ -91,6 +91,7 @@ StepKernel pick_kernel(int s1d, int tile) {
 struct dragon_batch {
     std::vector<dragon_grid*> members;
     dragon_batch_tuning tune{254, 0, 0, 32, 8, 1};
+    bool default_tiles = true;  // mhd_tiles was not set: build() chooses up to its value
     int s1d = -1;
     int prec = -1;  // the members' precision (0 FP64, 1 mixed)
     cudaStream_t stream = nullptr;
@@ -268,15 +269,16 @@ int build(dragon_batch* b) {
     CKB(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, 0));
     if (occ < 1) return fail(DRAGON_GPU_ECUDA, "batched step kernel cannot be resident");
     const int per_sm = b->tune.ctas_per_sm > 0 ? std::min(b->tune.ctas_per_sm, occ) : occ;
-    // Tiles of a 2D MHD phase per work item: the tuning's number, fewer where
-    // the members together have too few tiles of a phase for the resident CTAs
-    // (a phase of 8 grids of 80^2 to 160^2 took 100 items of eight tiles, one
+    // Tiles of a 2D MHD phase per work item: the tuning's number. Unless that
+    // was set, fewer where the members together have too few tiles of a phase
+    // for the resident CTAs (a phase of 8 grids of 80^2 to 160^2 took 100 items of eight tiles, one
     // after another, on 296 CTAs: 0.57 ms a step against 0.24 with two; 8
     // grids of 27^2 to 54^2: 0.36 against 0.11 with one)
     long long tiles = 0;
     for (dragon_grid* h : b->members)
         if (h->dim == 2) tiles += (long long)tiles_along(h->n[0] + 4, kTileI) * tiles_along(h->n[1] + 4, kTileJ);
-    const int group = (int)std::max<long long>(1, std::min<long long>(b->tune.mhd_tiles, tiles / (per_sm * sms)));
+    const int group = !b->default_tiles ? b->tune.mhd_tiles
+        : (int)std::max<long long>(1, std::min<long long>(b->tune.mhd_tiles, tiles / (per_sm * sms)));
     for (dragon_grid* h : b->members) insts.push_back(make_inst(h, b->tune.tile_1d, group, mixed));
     std::vector<int> fmembers;  // a mixed batch's 2D MHD members, in the fused launch's CTA order
     if (mixed) {
@@ -514,6 +516,7 @@ int dragon_gpu_batch_set_tuning(dragon_batch* b, const dragon_batch_tuning* t) {
         t->wave < 0 || t->wave > 64)
         return fail(DRAGON_GPU_EINVAL, "invalid batch tuning");
     b->tune = *t;
+    b->default_tiles = false;
     if (b->tune.mhd_tiles == 0) b->tune.mhd_tiles = 1;
     if (b->tune.wave == 0) b->tune.wave = 1;
     b->dirty = true;
@@ -582,11 +585,13 @@ int dragon_gpu_batch_autotune(dragon_batch* b, int steps, dragon_batch_tuning* b
         return 0;
     };
     const dragon_batch_tuning keep = b->tune;
+    const bool keep_default = b->default_tiles;
     dragon_batch_tuning win = keep;
     double win_ms = INFINITY;
     int rc = 0;
     auto trial = [&](const dragon_batch_tuning& t) -> int {
         b->tune = t;
+        b->default_tiles = false;
         b->dirty = true;
         dragon_batch_stats s{};
         int r = advance(b, steps, &s);
@@ -627,6 +632,7 @@ int dragon_gpu_batch_autotune(dragon_batch* b, int steps, dragon_batch_tuning* b
     free_snaps();
     win.graph_steps = keep.graph_steps;
     b->tune = win;
+    b->default_tiles = keep_default && win_ms == INFINITY;  // (no candidate ran)
     b->dirty = true;
     if (rc) return rc;
     if (best) *best = win;

@@ -42,7 +42,9 @@ typedef struct dragon_batch_tuning {
                          phase k queued with group g+1's phase k-1 (a group's intermediates are reused
                          while they are still in L2) */
     int graph_steps;  /* steps captured per CUDA graph */
-    int mhd_tiles;    /* 32 x 8 tiles of a 2D MHD phase per work item: 1, 2, 4 or 8 (0 reads as 1; default 8) */
+    int mhd_tiles;    /* 32 x 8 tiles of a 2D MHD phase per work item: 1, 2, 4 or 8 (0 reads as 1). A batch whose
+                         tuning was neither set nor tuned takes up to 8, fewer where its members have too few
+                         tiles to give every resident CTA an item (dragon_gpu_batch_get_tuning says 8 then) */
     int wave;         /* order 3: 2D MHD grids per wavefront group, 1..64 (0 reads as 1) */
 } dragon_batch_tuning;
 
