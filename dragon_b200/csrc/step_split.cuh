@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(256) k_sweep(Geo G, const double* __restrict__
         Prim<double> nw = W_at(l, c + 2);
         if (p >= 1 && p <= np - 2) {
             const Cons<double> fl = fget(l, c), fr = fget(l, c + 1);
-            nw = f64::corrected<false>(nw, c_mul<false>(c_sub<false>(fr, fl), dt_dx));
+            // minus the negated change: the sum and its zero's sign are those of the addition
+            nw = f64::corrected<false>(nw, c_mul<false>(c_sub<false>(fl, fr), -dt_dx));
             if (p == np - 2) nw = to_prim<false>(c_add<false>(to_cons<false>(nw), c_mul<false>(c_sub<false>(fr, fr), dt_dx)));
         }
         swap_axis<AX>(nw);
