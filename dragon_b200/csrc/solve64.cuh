@@ -502,7 +502,9 @@ __device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s
 // raises the flag. Only the side the contact leaves behind needs its star flux
 // and energy (SsL >= 0 implies SM >= 0, SsR <= 0 implies SM <= 0), so the
 // other side's star state comes first and leaves its velocity and field:
-// fewer values alive at a time (both sides whole spilled 700 bytes).
+// fewer values alive at a time (both sides whole spilled 700 bytes). Where an
+// inner wave stands on the face (SsL or SsR zero) the other side's star state
+// is not used, but an unphysical one still takes the face to HLLE.
 template <class C>
 __device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, C& ck) {
     const double Bx = (L.Bx + Rt.Bx) * 0.5;
@@ -549,7 +551,7 @@ __device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, C&
     const double aK = div(ab, s4 * sqK, ck), aO = div(ab, s4 * sqO, ck);
     const double SsL = SM - (left ? aK : aO), SsR = SM + (left ? aO : aK);
     const bool inner = !(SsL >= 0.0) && !(SsR <= 0.0);
-    if (inner) mhd_star<false, false>(O, sO, xO, SO, SM, dO, rhoO, pT, Bx, o, ck);
+    if (!(SsL > 0.0) && !(SsR < 0.0)) mhd_star<false, false>(O, sO, xO, SO, SM, dO, rhoO, pT, Bx, o, ck);
     mhd_star<false, true>(K, sK, xK, SK, SM, dK, rhoK, pT, Bx, k, ck);
     ck.raise(SsL >= 0.0 ? !left : SsR <= 0.0 && left);
     if (!inner) return k.F;
