@@ -325,10 +325,10 @@ __device__ __forceinline__ double exact_rho(double p, const Prim<double>& w, con
     if (p > w.p) return div(w.rho * (p + s.B), kGm1_Gp1 * p + w.p, ck);
     return w.rho * pow1(quot(p, s.rp), kGinv);
 }
-// the flux of the exact solution at x / t = 0
+// the flux of the exact solution at x / t = 0; ps: its star pressure
 template <class C>
 __device__ __forceinline__ Cons<double> exact(const Prim<double>& L, const Prim<double>& Rt, const ExactOpts& o,
-                                              FaceStats* st, C& ck) {
+                                              FaceStats* st, double& ps, C& ck) {
     ExactSide sL, sR;
     exact_side(L, sL, ck);
     exact_side(Rt, sR, ck);
@@ -364,6 +364,7 @@ __device__ __forceinline__ Cons<double> exact(const Prim<double>& L, const Prim<
     }
     ck.pos(p);
     ck.num(v);
+    ps = p;
     Prim<double> w;
     w.Bx = w.By = w.Bz = 0;
     if (fabs(v - 0.0) < 1e-12) {
@@ -615,7 +616,7 @@ __device__ __forceinline__ Cons<double> hlle_mhd(Prim<double> L, Prim<double> Rt
 // Flux.cpp:77-97); a test that fails or is close raises the flag.
 template <bool MHD, int SOLVER, class C>
 __device__ __forceinline__ void face_body(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
-                                          const ExactOpts& eo, Cons<double>& F, FaceStats* st, C& ck) {
+                                          const ExactOpts& eo, Cons<double>& F, FaceStats* st, double& ps, C& ck) {
     if constexpr (MHD) {
         if constexpr (SOLVER == RS_HLLE) F = hlle_mhd(L, Rt, ck);
         else F = hlld(L, Rt, ck);
@@ -625,7 +626,7 @@ __device__ __forceinline__ void face_body(const Prim<double>& L, const Prim<doub
         else if constexpr (SOLVER == RS_HLLE) F = hlle(L, Rt, sL, sR, ck);
         else if constexpr (SOLVER == RS_ROE) F = roe(L, Rt, sL, sR, ck);
         else if constexpr (SOLVER == RS_EXACT) {
-            F = exact(L, Rt, eo, st, ck);
+            F = exact(L, Rt, eo, st, ps, ck);
             sL.U = f64::to_cons<false>(L);
             sR.U = f64::to_cons<false>(Rt);
         } else F = hllc(L, Rt, sL, sR, ck);
@@ -637,26 +638,48 @@ __device__ __forceinline__ void face_body(const Prim<double>& L, const Prim<doub
         }
     }
 }
-template <bool MHD, int SOLVER, bool AGAIN>
+// The exact solver's face while its solves are logged: false if it raises the
+// flag (then nothing is logged here).
+template <bool LOCAL>
+__device__ __noinline__ bool exact_logged(const Prim<double>* LR, double dt_dx, const ExactOpts* eo, Cons<double>* F,
+                                          FaceStats* st) {
+    Flag<LOCAL> ck;
+    FaceStats s = *st;
+    double ps;
+    face_body<false, RS_EXACT>(LR[0], LR[1], dt_dx, *eo, *F, &s, ps, ck);
+    if (ck.bad) return false;
+    // (without a flag both states and the pressure are positive and finite)
+    if (s.exact_calls != st->exact_calls && s.cap_hits == st->cap_hits)
+        newton_log_push(eo->log, LR[0].rho, LR[0].vx, LR[0].p, LR[1].rho, LR[1].vx, LR[1].p, ps,
+                        s.newton_iters - st->newton_iters);
+    *st = s;
+    return true;
+}
+template <bool MHD, int SOLVER, bool AGAIN, bool LOCAL>
 __device__ __noinline__ bool face_slow(const Prim<double>* LR, double dt_dx, const ExactOpts* eo, Cons<double>* F,
                                        FaceStats* st) {
     if constexpr (AGAIN) {
         Flag<true> ck;
         FaceStats s = *st;
-        face_body<MHD, SOLVER>(LR[0], LR[1], dt_dx, *eo, *F, &s, ck);
+        double ps;
+        face_body<MHD, SOLVER>(LR[0], LR[1], dt_dx, *eo, *F, &s, ps, ck);
         if (!ck.bad) {
             *st = s;
             return true;
         }
-        return face_slow<MHD, SOLVER, false>(LR, dt_dx, eo, F, st);
+        return face_slow<MHD, SOLVER, false, LOCAL>(LR, dt_dx, eo, F, st);
     } else {
+        if constexpr (!MHD && SOLVER == RS_EXACT)
+            if (eo->log.rows && eo->guess == GUESS_MEAN && exact_logged<LOCAL>(LR, dt_dx, eo, F, st)) return true;
         return face_flux_x<MHD, SOLVER, double>(LR[0], LR[1], dt_dx, *eo, *F, st);
     }
 }
 
 // The flux along x of the states on both sides of a face, as face_flux_x. MHD
 // HLL is rare and takes the plain routine, and so does the exact solver with
-// another guess than the mean or while its solves are logged.
+// another guess than the mean. While its solves are logged they run out of line
+// (a branch to the log behind every exact solve here cost 1.8 %, its star
+// pressure kept to the end of the face 1.2 %: 3D blast 110 x 87 x 93).
 template <bool MHD, int SOLVER, bool LOCAL = false>
 __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<double>& Rt, double dt_dL,
                                             const ExactOpts& eo, Cons<double>& F, FaceStats* st) {
@@ -666,9 +689,10 @@ __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<do
         constexpr bool kExact = !MHD && SOLVER == RS_EXACT;
         Flag<LOCAL> ck;
         FaceStats s = *st;
-        const bool plain = kExact && (eo.guess != GUESS_MEAN || eo.log.rows);
-        if (!plain) {
-            face_body<MHD, SOLVER>(L, Rt, dt_dL, eo, F, &s, ck);
+        const bool aside = kExact && (eo.guess != GUESS_MEAN || eo.log.rows);
+        if (!aside) {
+            double ps;
+            face_body<MHD, SOLVER>(L, Rt, dt_dL, eo, F, &s, ps, ck);
             if (!ck.bad) {
                 if constexpr (kExact) *st = s;
                 return true;
@@ -678,7 +702,7 @@ __device__ __forceinline__ bool face_flux_x(const Prim<double>& L, const Prim<do
         Cons<double> G;
         const ExactOpts e = eo;
         FaceStats t = *st;
-        const bool ok = face_slow<MHD, SOLVER, !LOCAL && !kExact>(LR, dt_dL, &e, &G, &t);
+        const bool ok = face_slow<MHD, SOLVER, !LOCAL && !kExact, LOCAL>(LR, dt_dL, &e, &G, &t);
         *st = t;
         F = G;
         return ok;
