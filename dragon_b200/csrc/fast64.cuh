@@ -54,6 +54,14 @@ namespace f64 {
 // (quot). A numerator that is infinite, NaN or too large needs no test of its
 // own there: it makes the quotient NaN or huge, and the sum, pressure, energy
 // or radicand it goes into has a test.
+//
+// In centimetres and seconds some divisors are far above 2^50. A quotient of
+// its own (div) takes divisors below 2^102: its remainders are exact down to
+// quotients of 2^-1022, where the second part of a reciprocal has lost its
+// bits. The others are a WideRec: a cell width, a pressure, the square of a
+// speed, a density times one or two speeds.
+
+constexpr unsigned kNumFloor = (1023u - 920u) << 20;  // 2^-920
 
 // The flag of one face, cell or state. With LOCAL the quotients of small
 // numerators are divided by the plain operator on the spot: a branch per group
@@ -64,10 +72,11 @@ template <bool LOCAL>
 struct Flag {
     static constexpr bool kLocal = LOCAL;
     bool bad = false;
-    // |x| in [2^-120, 2^50)
+    // |x| in [2^-120, 2^MAX)
+    template <unsigned MAX = 50>
     __device__ __forceinline__ void den(double x) {
         const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
-        bad |= u - ((1023u - 120u) << 20) >= (170u << 20);
+        bad |= u - ((1023u - 120u) << 20) >= ((MAX + 120u) << 20);
     }
     // x in [2^-120, 2^50)
     __device__ __forceinline__ void posden(double x) {
@@ -81,20 +90,23 @@ struct Flag {
     __device__ __forceinline__ void fin(double x) {
         bad |= ((unsigned)__double2hiint(x) & 0x7fffffffu) >= ((1023u + 850u) << 20);
     }
-    // x == 0 or |x| in [2^-920, 2^850)
-    __device__ __forceinline__ void num(double x) {
+    // x == 0 or |x| in [lo, 2^1770 lo), lo a high word (2^-920, or what num_floor gives)
+    __device__ __forceinline__ void num(double x, unsigned lo = kNumFloor) {
         const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
         const unsigned z = u | (unsigned)__double2loint(x);
-        bad |= (u - ((1023u - 920u) << 20) >= (1770u << 20)) && z != 0u;
+        bad |= (u - lo >= (1770u << 20)) && z != 0u;
     }
     __device__ __forceinline__ void raise(bool c) { bad |= c; }
 };
 using Chk = Flag<false>;
 
-// 0 < |x| < 2^-920
-__device__ __forceinline__ bool tiny(double x) {
+// max(2^-920, 2^-970 |b|) as a high word, of that of |b|: the smallest numerator
+// for a divisor of any size.
+__device__ __forceinline__ unsigned floor_of(unsigned b) { return max(b, (1023u + 50u) << 20) - (970u << 20); }
+// 0 < |x| < lo
+__device__ __forceinline__ bool tiny(double x, unsigned lo) {
     const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    return u < ((1023u - 920u) << 20) && (u | (unsigned)__double2loint(x)) != 0u;
+    return u < lo && (u | (unsigned)__double2loint(x)) != 0u;
 }
 static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
 
@@ -133,6 +145,18 @@ __device__ __forceinline__ PosRec posrec(double b, C& ck) {
     ck.posden(b);
     return PosRec{rec_of(b)};
 }
+// of a divisor in [2^-120, 2^400), whose numerators' floor goes with it: two
+// integer instructions (for every divisor 0.5 to 1.8 % of a step)
+struct WideRec : Rec {};
+template <class C>
+__device__ __forceinline__ WideRec widerec(double b, C& ck) {
+    ck.template den<400>(b);
+    return WideRec{rec_of(b)};
+}
+__device__ __forceinline__ unsigned num_floor(const Rec&) { return kNumFloor; }
+__device__ __forceinline__ unsigned num_floor(const WideRec& r) {
+    return floor_of((unsigned)__double2hiint(r.b) & 0x7fffffffu);
+}
 
 // The sign a zero quotient takes (the corrections lose it); others have it already.
 __device__ __forceinline__ double signed_as(double q, double a, double b) {
@@ -156,9 +180,10 @@ __device__ __forceinline__ double quot(double a, const Rec& r) {
 // a / r.b for several values at once.
 template <class Q, class C, class... D>
 __device__ __forceinline__ void quots(const Q& r, C& ck, D&... a) {
+    const unsigned lo = num_floor(r);
     if constexpr (C::kLocal) {
         (ck.fin(a), ...);
-        const bool small = (tiny(a) || ...);
+        const bool small = (tiny(a, lo) || ...);
         const double n[sizeof...(D)] = {a...};
         ((a = signed_as(quot(a, r), a, r)), ...);
         if (small) {
@@ -166,7 +191,7 @@ __device__ __forceinline__ void quots(const Q& r, C& ck, D&... a) {
             ((a = div_plain(n[k++], r.b)), ...);
         }
     } else {
-        (ck.num(a), ...);
+        (ck.num(a, lo), ...);
         ((a = signed_as(quot(a, r), a, r)), ...);
     }
 }
@@ -181,7 +206,7 @@ __device__ __forceinline__ double div_of(double a, double b) {
 template <class C>
 __device__ __forceinline__ double div(double a, double b, C& ck) {
     ck.num(a);
-    ck.den(b);
+    ck.template den<102>(b);
     return signed_as(div_of(a, b), a, b);
 }
 
@@ -309,9 +334,9 @@ __device__ __forceinline__ Widths widths(int dim, double dx, double dy, double d
     Widths d;
     ck.raise(!(dx > 1e-14 && dy > 1e-14 && (dim < 3 || dz > 1e-14)));  // cfl_speed leaves these axes out
     d.three = dim > 2;
-    d.x = rec(dx, ck);
-    d.y = rec(dy, ck);
-    d.z = rec(d.three ? dz : 1.0, ck);
+    d.x = widerec(dx, ck);  // (of numerators that are speeds: above 2^-275)
+    d.y = widerec(dy, ck);
+    d.z = widerec(d.three ? dz : 1.0, ck);
     d.bad = ck.bad;
     return d;
 }

@@ -14,11 +14,13 @@ namespace dgpu {
 namespace f64 {
 
 // n / d for slopes of one sign (on), 0 otherwise. With n at least 2^-900 the
-// divisor may be smaller than elsewhere.
-template <class C>
+// divisor may lie in [2^-450, 2^120) (div_of needs no more than a normal
+// quotient). WIDE: up to 2^400, with n at least 2^-950 d, for a sum of squares.
+template <bool WIDE, class C>
 __device__ __forceinline__ double slope_quot(double n, double d, bool on, C& ck) {
     const unsigned un = (unsigned)__double2hiint(n) & 0x7fffffffu, ud = (unsigned)__double2hiint(d) & 0x7fffffffu;
-    const bool odd = on && (un - ((1023u - 900u) << 20) >= (1800u << 20) || ud - ((1023u - 450u) << 20) >= (500u << 20));
+    const unsigned lo = WIDE ? floor_of(ud) + (20u << 20) : (1023u - 900u) << 20;
+    const bool odd = on && (un - lo >= (1800u << 20) || ud - ((1023u - 450u) << 20) >= ((WIDE ? 850u : 570u) << 20));
     if constexpr (C::kLocal) {
         if (odd) return div_plain(n, d);
     } else {
@@ -32,9 +34,9 @@ __device__ __forceinline__ double limit1(int lim, double a, double b, C& ck) {
     switch (lim) {
         case LIM_MC: return lim_mc(a, b);
         // the plain form divides (2 a) b by a + b unless a b <= 0
-        case LIM_VANLEER: return slope_quot((2.0 * a) * b, a + b, !(a * b <= 0.0), ck);
+        case LIM_VANLEER: return slope_quot<false>((2.0 * a) * b, a + b, !(a * b <= 0.0), ck);
         case LIM_SUPERBEE: return lim_superbee(a, b);
-        case LIM_VANALBADA: return slope_quot((a * b) * (a + b), a * a + b * b, !(a * b <= 0.0), ck);
+        case LIM_VANALBADA: return slope_quot<true>((a * b) * (a + b), a * a + b * b, !(a * b <= 0.0), ck);
         default: return lim_minmod(a, b);
     }
 }
@@ -255,7 +257,7 @@ __device__ __forceinline__ Cons<double> roe(const Prim<double>& L, const Prim<do
     const double _a = root(kGm1 * (_H - V2 * 0.5), ck);
     const double dp = Rt.p - L.p, ra = _rho * _a, du = Rt.vx - L.vx;
     // (2 a) a is exactly twice a a, so all three quotients share 1 / (a a)
-    const Rec r2 = rec(_a * _a, ck);
+    const WideRec r2 = widerec(_a * _a, ck);
     double q0 = dp - ra * du, q1 = dp, q4 = dp + ra * du;
     quots(r2, ck, q0, q1, q4);
     const double al0 = 0.5 * q0, al1 = (Rt.rho - L.rho) - q1, al2 = _rho * (Rt.vy - L.vy), al3 = _rho * (Rt.vz - L.vz),
@@ -305,12 +307,12 @@ __device__ __forceinline__ void exact_side(const Prim<double>& w, ExactSide& s, 
     s.A = quot(k2_Gp1, r);
     s.B = kGm1_Gp1 * w.p;
     s.ra = w.rho * s.a;
-    s.rp = rec(w.p, ck);
+    s.rp = widerec(w.p, ck);  // (here and in exact_f of numerators above 2^-460)
 }
 template <bool DERIV, class C>
 __device__ __forceinline__ double exact_f(double p, const Prim<double>& w, const ExactSide& s, double& df, C& ck) {
     if (p > w.p) {
-        const Rec r = rec(s.B + p, ck);
+        const Rec r = widerec(s.B + p, ck);
         const double q = root(quot(s.A, r), ck), d = p - w.p;
         if constexpr (DERIV) df = q * (1.0 - 0.5 * quot(d, r));
         return d * q;
@@ -460,7 +462,7 @@ __device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s
         const double bb = (Bx * Bx) * k1_4pi;
         const double den = x * d.b - bb, num = x * (SK - K.vx) - bb, dv = SM - K.vx;
         ck.raise(!(fabs(den) >= 1e-12));
-        const Rec q = rec(den, ck);
+        const WideRec q = widerec(den, ck);  // a density times two speeds
         u.Bx = Bx;
         u.By = K.By * num;
         u.Bz = K.Bz * num;
@@ -522,7 +524,7 @@ __device__ __forceinline__ Cons<double> hlld(Prim<double> L, Prim<double> Rt, C&
         const double pTL = L.p + b2_of(L) * k1_8pi, pTR = Rt.p + b2_of(Rt) * k1_8pi;
         xL = L.rho * (SL - L.vx);
         xR = Rt.rho * (SR - Rt.vx);
-        const Rec rx = rec(xR - xL, ck);
+        const WideRec rx = widerec(xR - xL, ck);
         SM = (xR * Rt.vx - xL * L.vx) - (pTR - pTL);
         quots(rx, ck, SM);
         pT = quot(xR * pTL - xL * pTR + xL * xR * (Rt.vx - L.vx), rx);
