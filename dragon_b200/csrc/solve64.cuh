@@ -461,12 +461,13 @@ __device__ __forceinline__ void mhd_star(const Prim<double>& K, const MhdSide& s
     } else {
         const double bb = (Bx * Bx) * k1_4pi;
         const double den = x * d.b - bb, num = x * (SK - K.vx) - bb, dv = SM - K.vx;
-        ck.raise(!(fabs(den) >= 1e-12));
-        const WideRec q = widerec(den, ck);  // a density times two speeds
+        // a density times two speeds: always below 1e-12 in the units of thin gas
+        const bool degen = fabs(den) < 1e-12;
+        const WideRec q = widerec(degen ? 1.0 : den, ck);
         u.Bx = Bx;
-        u.By = K.By * num;
-        u.Bz = K.Bz * num;
-        double ty = (K.By * Bx) * dv, tz = (K.Bz * Bx) * dv;
+        u.By = degen ? K.By : K.By * num;
+        u.Bz = degen ? K.Bz : K.Bz * num;
+        double ty = degen ? 0.0 : (K.By * Bx) * dv, tz = degen ? 0.0 : (K.Bz * Bx) * dv;
         quots(q, ck, u.By, u.Bz, ty, tz);
         vy = K.vy - ty * k1_4pi;
         vz = K.vz - tz * k1_4pi;

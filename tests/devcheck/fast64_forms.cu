@@ -189,6 +189,13 @@ int forms_face(int solver, int local, long long n, const double* L, const double
     return done(O, out, 28 * n);
 }
 
+int forms_mhd_face(int solver, long long n, const double* L, const double* R, double dt_dx, double* out) {
+    Buf A(L, n * 8), B(R, n * 8), O(nullptr, 28 * n);
+    if (solver == RS_HLLE) k_face<true, RS_HLLE, false><<<grid_of(n), 128>>>(n, A.p, B.p, dt_dx, O.p);
+    else k_face<true, RS_HLLD, false><<<grid_of(n), 128>>>(n, A.p, B.p, dt_dx, O.p);
+    return done(O, out, 28 * n);
+}
+
 int forms_muscl(int local, int lim, long long n, const double* L, const double* C, const double* R, double dt_dx, double* out) {
     Buf A(L, n * 5), B(C, n * 5), D(R, n * 5), O(nullptr, 34 * n);
     if (local) k_muscl<true><<<grid_of(n), 128>>>(n, lim, A.p, B.p, D.p, dt_dx, O.p);

@@ -25,8 +25,8 @@ UNITS = {
     "stellar interior": (150.0, 6e7, 1e8),
     "white dwarf": (1e7, 5e8, 1e5),
 }
-MHD_UNITS = {"order one": (1.0, 1.0, 0.01), "photosphere": (3e-7, 8e5, 1e7), "stellar interior": (150.0, 6e7, 1e8),
-             "neutron star crust": (1e11, 3e9, 1e4)}
+MHD_UNITS = {"order one": (1.0, 1.0, 0.01), "interstellar gas": (2e-24, 1e5, 3e18), "photosphere": (3e-7, 8e5, 1e7),
+             "stellar interior": (150.0, 6e7, 1e8), "neutron star crust": (1e11, 3e9, 1e4)}
 
 
 @pytest.fixture(scope="module")
@@ -39,6 +39,7 @@ def lib(tmp_path_factory):
     i, n, d = ctypes.c_int, ctypes.c_longlong, ctypes.c_double
     L.forms_arith.argtypes = [i, n, D, D, D, ctypes.POINTER(i)]
     L.forms_face.argtypes = [i, i, n, D, D, d, D]
+    L.forms_mhd_face.argtypes = [i, n, D, D, d, D]
     L.forms_muscl.argtypes = [i, i, n, D, D, D, d, D]
     L.forms_cell.argtypes = [i, i, i, n, D, D, D]
     L.forms_flags.argtypes = [i, i, i, n, D, D, D, d, d, ctypes.POINTER(i)]
@@ -100,6 +101,19 @@ def test_exact_solver_counters(lib, local):
     done = same & (out[1, :, 8] == 1) & (out[1, :, 13] == 0)
     scale = np.abs(out[1, done, :8]).max(1, keepdims=True)
     assert (np.abs(out[0, done, :8] - out[1, done, :8]) / scale).max() < 1e-13
+
+
+@pytest.mark.parametrize("units", list(MHD_UNITS))
+@pytest.mark.parametrize("solver", [HLLD, HLLE])
+def test_mhd_faces(lib, solver, units):
+    rng = np.random.default_rng(41 + solver)
+    w = states(rng, N, True)
+    rho, v, _ = MHD_UNITS[units]
+    L, R = in_units(w, rho, v), in_units(neighbour(rng, w), rho, v)
+    out = np.zeros((2, N, 14))
+    assert lib.forms_mhd_face(solver, N, p(L), p(R), 0.2 / v, p(out)) == 0
+    ok = same_bits(out[0], out[1]).all(1)
+    assert ok.all(), (L[~ok][:3], R[~ok][:3], out[:, ~ok][:, :3])
 
 
 @pytest.mark.parametrize("units", ["order one", "cluster gas at 1e8 K"])
