@@ -18,15 +18,25 @@ constexpr int k2dTI = 16, k2dTJ = 24, k2dNT = 256;
 // for its arithmetic, so smaller grids take smaller tiles: 6 x 30 cells, whose
 // 256 half states are one round of the threads (faces and corrections two),
 // and 6 x 14, whose every phase is one round (128 half states, 232 and 188
-// faces, 208 corrections, 84 updates). Step times in us, 6 x 14 / 6 x 30 / 14 x
-// 26 cells: 96^2 22.6 / 24.7 / 32.9, 128^2 25.6 / 25.7 / 33.9, 200^2 35.6 / 31.0
-// / 33.1, 320^2 61.6 / 51.1 / 56.2, 400^2 85 / 68.5 / 68.6, 512^2 128 / 96 / 82.
-// Hence the lines: 6 x 14 up to one CTA per SM, 6 x 30 up to five.
+// faces, 208 corrections, 84 updates). Step times in us (CTAs), shear layer:
+//          6 x 14        6 x 30       16 x 24
+//  96^2   17.5 (112)   19.1  (64)   27.2  (24)
+// 128^2   18.9 (220)   20.5 (110)   27.8  (48)
+// 160^2   26.0 (324)   24.9 (162)   27.4  (70)
+// 256^2   40.1 (817)   33.9 (387)   38.5 (176)
+// 300^2   50.2         40.7 (500)   38.7 (247)
+// 320^2   54.5         43.5 (594)   38.6 (280)
+// 350^2   60.1         48.8 (708)   51.6 (330)
+// 384^2   74.0         55.4 (832)   52.3 (384)
+// Hence the lines: 6 x 14 while its CTAs are all resident (two per SM), 6 x 30
+// up to three per SM, and up to five where the large tiles need a second wave.
 enum Tile2D { kTile16x24, kTile6x30, kTile6x14 };
+constexpr long long kSms = 148;  // of a B200
 static Tile2D pick_tile(const Geo& G) {
     auto ctas = [&](int ti, int tj) { return (long long)((G.n[0] + ti - 1) / ti) * ((G.n[1] + tj - 1) / tj); };
-    if (ctas(6, 14) <= 148) return kTile6x14;
-    if (ctas(6, 30) <= 148 * 5) return kTile6x30;
+    if (ctas(6, 14) <= 2 * kSms) return kTile6x14;
+    const long long mid = ctas(6, 30);
+    if (mid <= 3 * kSms || (mid <= 5 * kSms && ctas(k2dTI, k2dTJ) > 2 * kSms)) return kTile6x30;
     return kTile16x24;
 }
 
