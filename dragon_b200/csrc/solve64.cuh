@@ -1,6 +1,7 @@
 // FP64 reconstruction and Riemann solvers of the step kernels on the
 // branch-free divisions of fast64.cuh: the same results as muscl() and
-// face_flux() bit for bit. Each first computes without a branch per division
+// face_flux() bit for bit, but for the exact solver, whose star pressure may
+// differ in its last places (exact_f). Each first computes without a branch per division
 // and raises a flag on anything out of the ordinary (an operand out of range,
 // an unphysical or borderline state, a fallback of the solver); the face or
 // cell is then repeated out of line, in the end by the plain routine.
